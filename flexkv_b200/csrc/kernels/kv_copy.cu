@@ -1,15 +1,18 @@
 // Paged KV gather/scatter kernels (see kv_copy.h for the addressing model).
 //
-// Engine 0 — bulk-copy pipeline. Each persistent CTA is one warp that drives
-// a ring of shared-memory stages through the TMA unit: lane 0 issues a 1-D
-// bulk load (global -> shared, completion on an mbarrier) for tiles up to
-// LOOKAHEAD ahead, and as each tile lands issues the matching bulk store
-// (shared -> global). Either side may be mapped host memory, so the same
-// pipeline does GPU->host and host->GPU with no SM load/store instructions
-// on the data and no registers holding payload; the other lanes only
-// prefetch block ids. Host reads need many bytes in flight to cover the PCIe
-// round trip, so host->GPU runs with LOOKAHEAD = STAGES-1; GPU->host keeps
-// half of the ring for queued posted writes.
+// Engine 0 — bulk-copy pipeline. A persistent CTA runs W independent one-warp pipelines, each with its own ring
+// of shared-memory stages driven through the TMA unit: lane 0 issues a 1-D bulk load (global -> shared,
+// completion on an mbarrier) for tiles up to LOOKAHEAD ahead, and as each tile lands issues the matching bulk
+// store (shared -> global). Either side may be mapped host memory, so the same pipeline does GPU->host and
+// host->GPU with no SM load/store instructions on the data and no registers holding payload. The addresses of
+// the next 32 tiles are computed by the 32 lanes at once and handed to lane 0 through shared memory.
+//
+// What bounds it: against the host, the link, from two to four CTAs on; between two places in HBM, the bytes a CTA
+// can keep in flight (192 KiB, about 48 GB/s per CTA). Before, one warp per CTA computed the addresses tile by tile
+// and took 0.8 us per tile whatever its size. Measured on B200, GB/s before -> now, 8 CTAs:
+//   4 KiB chunks GPU->host 40 -> 52.5, host->GPU 41 -> 51.3 (16 CTAs 52.4 -> 52.5 / 39 -> 51.3); 1 KiB 10 -> 52.5
+//   within HBM: 4 KiB chunks 40 -> 378, 32 KiB 160 -> 391; 64 CTAs 300 -> 2470 and 1180 -> 2570
+//   one op of 2 MiB in 32 KiB chunks: GPU->host 54 -> 50 us
 //
 // Engine 1 — SIMT vector copy, warp per tile, 16/8/4/1-byte lanes with an
 // 8-deep unrolled load batch. It serves chunks whose size or alignment rules
@@ -74,43 +77,56 @@ __device__ __forceinline__ bool ids_in_range(const KvCopyParams& p, int64_t g, i
   return ok;
 }
 
-// Layer-major launches run a second warp per CTA whose only job is the per-layer publication: fences, the
-// counter atomic and the system-scope flag store issued by the copy thread itself would wait for that
-// thread's loads in flight and drain the pipeline at every layer boundary. The copy thread only waits for
-// its bulk stores and posts "layers [0, n) done" to a shared-memory mailbox.
-template <int STAGES, int LOOKAHEAD>
-__global__ void __launch_bounds__(64, 1)
+// Descriptors of the tiles a pipeline is working on: written by all lanes 32 tiles at a time, read by lane 0.
+// Between the oldest tile whose store is still to be issued and the newest one decoded lie at most
+// LOOKAHEAD + 32 <= 63 tiles.
+constexpr int kDescRing = 64;
+struct TileDesc {
+  uint64_t src, dst;
+  uint32_t bytes;   // 0 = skipped
+  int32_t major;    // layer-major launches: layer (relative) of the tile
+};
+
+// Layer-major launches run one more warp per CTA whose only job is the per-layer publication: fences, the
+// counter atomic and the system-scope flag store issued by a copy warp itself would wait for that warp's loads
+// in flight and drain the pipeline at every layer boundary. The copy warps only wait for their bulk stores and
+// post "layers [0, n) done" to a shared-memory mailbox each; the CTA has finished what all of them have.
+template <int W, int STAGES, int LOOKAHEAD>
+__global__ void __launch_bounds__(32 * (W + 1), 1)
 kv_copy_bulk_kernel(const __grid_constant__ KvCopyParams p, int tile_bytes, int tiles_per_chunk) {
   static_assert(LOOKAHEAD >= 1 && LOOKAHEAD < STAGES, "lookahead must leave one stage for stores");
   static_assert(STAGES <= 32, "stage phases are kept in one 32-bit mask");
-  extern __shared__ __align__(128) uint8_t ring[];
-  __shared__ __align__(8) uint64_t full[STAGES];
-  __shared__ uint64_t s_dst[STAGES];
-  __shared__ uint32_t s_bytes[STAGES];
-  __shared__ int32_t s_layer[STAGES];   // layer-major launches: layer (relative) of the tile in the stage
-
-  __shared__ int s_layers_done;         // mailbox: this CTA finished (stores included) layers [0, n)
-  const int lane = threadIdx.x & 31;
+  static_assert(LOOKAHEAD + 32 < kDescRing, "descriptor ring");
+  extern __shared__ __align__(128) uint8_t ring_all[];
+  __shared__ __align__(8) uint64_t full_all[W][STAGES];
+  __shared__ TileDesc desc_all[W][kDescRing];
+  __shared__ int s_layers_done[W];      // mailboxes: this warp finished (stores included) layers [0, n)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
+    for (int w = 0; w < W; ++w) {
 #pragma unroll
-    for (int s = 0; s < STAGES; ++s) ptx::mbar_init(&full[s], 1);
+      for (int s = 0; s < STAGES; ++s) ptx::mbar_init(&full_all[w][s], 1);
+      s_layers_done[w] = 0;
+    }
     ptx::fence_mbar_init();
-    s_layers_done = 0;
   }
   __syncthreads();
-  if (threadIdx.x >= 32) {
+  const bool signalling = p.layer_major && p.done_counter != nullptr;
+  if (warp == W) {
     // ---- signaller warp (present only on layer-major launches with signalling)
-    if (lane != 0 || !p.layer_major || p.done_counter == nullptr) return;
+    if (lane != 0 || !signalling) return;
     int sig = 0;
     const uint64_t t0 = ptx::globaltimer_ns();
     while (sig < p.num_layers) {
-      const int d = *reinterpret_cast<volatile int*>(&s_layers_done);
+      int d = p.num_layers;
+#pragma unroll
+      for (int w = 0; w < W; ++w) d = min(d, *reinterpret_cast<volatile int*>(&s_layers_done[w]));
       if (d > sig) {
-        __threadfence_block();            // acquire side of the mailbox
+        __threadfence_block();            // acquire side of the mailboxes
         signal_layers(p, sig, d);
         sig = d;
       } else {
-        if (ptx::globaltimer_ns() - t0 > kSignalBudgetNs) {   // the copy warp always posts the last layer; belt and braces
+        if (ptx::globaltimer_ns() - t0 > kSignalBudgetNs) {   // the copy warps always post the last layer; belt and braces
           if (p.status) report_status(p.status, KV_ERR_WAIT_EXPIRED);
           return;
         }
@@ -119,110 +135,108 @@ kv_copy_bulk_kernel(const __grid_constant__ KvCopyParams p, int tile_bytes, int 
     }
     return;
   }
-  const bool has_signaller = blockDim.x > 32;
+  uint8_t* const ring = ring_all + (size_t)warp * STAGES * tile_bytes;
+  uint64_t* const full = full_all[warp];
+  TileDesc* const desc = desc_all[warp];
 
-  // span = tiles per major unit (a pair, or a layer when layer-major); all counts fit 32 bits
+  // span = tiles per major unit (a pair, or a layer when layer-major); counts per pipeline fit 32 bits
   const int32_t n_major = p.layer_major ? p.num_layers : p.num_pairs;
   const int32_t span = (p.layer_major ? p.num_pairs : p.num_layers) * p.kv_dim * tiles_per_chunk;
   const int64_t total = (int64_t)span * n_major;
-  const int64_t first = blockIdx.x, step = gridDim.x;
-  const int64_t n_mine = first < total ? (total - first + step - 1) / step : 0;
-  // the walk (major, r) advances by `step` tiles per iteration without divisions
-  const int32_t step_q = (int32_t)(step / span), step_r = (int32_t)(step % span);
-  int32_t major = (int32_t)(first / span), r = (int32_t)(first % span);
-
-  // Block ids are fetched 32 pairs at a time, one pair per lane, and the next
-  // window is requested as soon as the current one becomes active, so the
-  // round trip to (possibly host-resident) id arrays is off the issue path.
-  int32_t cur_w = -1;
-  int64_t cur_g = 0, cur_c = 0, nxt_g = 0, nxt_c = 0;
-  auto load_window = [&](int32_t w, int64_t& g, int64_t& c) {
-    const int64_t i = ((int64_t)w << 5) + lane;
-    if (i < p.num_pairs) {
-      g = __ldg(p.gpu_blocks + i);
-      c = __ldg(p.cpu_blocks + i);
-    }
+  // consecutive tiles go to different CTAs first, so that a small op uses all of them
+  const int64_t first = (int64_t)warp * gridDim.x + blockIdx.x, step = (int64_t)gridDim.x * W;
+  const int32_t n_mine = first < total ? (int32_t)((total - first + step - 1) / step) : 0;
+  // this lane decodes tiles lane, lane + 32, ... of the pipeline; (major, r) advances without divisions
+  const int64_t step32 = step * 32;
+  const int32_t step_q = (int32_t)(step32 / span), step_r = (int32_t)(step32 % span);
+  const int64_t t_lane = first + lane * step;
+  int32_t major = (int32_t)(t_lane / span), r = (int32_t)(t_lane % span);
+  TilePos pos{0, 0, 0, 0};
+  int64_t gblk = 0, cblk = 0;
+  // block ids may live in host memory: those of the next batch are requested while this one is being moved
+  auto fetch = [&](int32_t idx) {
+    if (idx >= n_mine) return;
+    pos = decode_tile(p, major, r, tiles_per_chunk);
+    gblk = __ldg(p.gpu_blocks + pos.pair);
+    cblk = __ldg(p.cpu_blocks + pos.pair);
   };
+  fetch(lane);
 
   int err = 0;
   int dead = 0;          // set after an expired wait: stop issuing, drain, leave
   uint32_t phases = 0;   // lane 0: parity of the next completion of each stage's barrier
-  int32_t signalled = 0; // lane 0, layer-major: layers [0, signalled) already reported by this CTA
+  int ld_st = 0, st_st = 0;   // lane 0: stage of the next load / of the next store
+  int32_t signalled = 0; // lane 0, layer-major: layers [0, signalled) already posted by this warp
 
-  for (int64_t it = 0; it < n_mine + LOOKAHEAD && !dead; ++it) {
-    const int64_t j = it - LOOKAHEAD;
-    if (j >= 0 && lane == 0) {
-      const int st = (int)(j % STAGES);
-      const uint32_t bytes = s_bytes[st];
-      if (p.layer_major && p.done_counter && s_layer[st] > signalled) {
-        // first store of a later layer: everything this CTA owned in the earlier layers is committed;
-        // drain those stores (the loads in flight are unaffected) and report the layers
-        ptx::bulk_wait<0>();
-        if (has_signaller) {
-          __threadfence_block();
-          *reinterpret_cast<volatile int*>(&s_layers_done) = s_layer[st];
-        } else {
-          signal_layers(p, signalled, s_layer[st]);
-        }
-        signalled = s_layer[st];
+  const int32_t n_steps = n_mine > 0 ? n_mine + LOOKAHEAD : 0;
+  for (int32_t base = 0; base < n_steps; base += 32) {
+    if (base + lane < n_mine) {
+      TileDesc d{0, 0, 0, major};
+      if (ids_in_range(p, gblk, cblk, err)) {
+        const TileAddr a = tile_addr(p, pos, gblk, cblk, tile_bytes);
+        d.src = p.h2d ? a.cpu : a.gpu;
+        d.dst = p.h2d ? a.gpu : a.cpu;
+        d.bytes = a.bytes;
       }
-      if (bytes) {
-        if (ptx::mbar_wait_bounded(&full[st], (phases >> st) & 1u, kWaitBudgetNs)) {
-          phases ^= 1u << st;
-          ptx::bulk_s2g(reinterpret_cast<void*>(s_dst[st]), ring + (size_t)st * tile_bytes, bytes);
-        } else {
-          err |= KV_ERR_WAIT_EXPIRED;
-        }
-      }
-      ptx::bulk_commit();  // one group per tile (possibly empty) keeps the wait arithmetic uniform
-    }
-    dead = __shfl_sync(0xffffffffu, (err & KV_ERR_WAIT_EXPIRED) ? 1 : 0, 0);
-    if (dead) break;
-
-    if (it < n_mine) {
-      const TilePos t = decode_tile(p, major, r, tiles_per_chunk);
-      const int32_t w = t.pair >> 5;
-      if (w != cur_w) {
-        if (w == cur_w + 1 && cur_w >= 0) { cur_g = nxt_g; cur_c = nxt_c; }
-        else load_window(w, cur_g, cur_c);
-        cur_w = w;
-        load_window(w + 1, nxt_g, nxt_c);
-      }
-      const int64_t gblk = __shfl_sync(0xffffffffu, cur_g, t.pair & 31);
-      const int64_t cblk = __shfl_sync(0xffffffffu, cur_c, t.pair & 31);
-      if (lane == 0) {
-        const int st = (int)(it % STAGES);
-        // the stage was last used by tile it-STAGES; all but the newest
-        // STAGES-LOOKAHEAD store groups must have finished reading smem
-        if (it >= STAGES) ptx::bulk_wait_read<STAGES - LOOKAHEAD>();
-        TileAddr a{0, 0, 0};
-        if (ids_in_range(p, gblk, cblk, err)) a = tile_addr(p, t, gblk, cblk, tile_bytes);
-        s_bytes[st] = a.bytes;
-        s_layer[st] = major;
-        if (a.bytes) {
-          s_dst[st] = p.h2d ? a.gpu : a.cpu;
-          ptx::mbar_expect_tx(&full[st], a.bytes);
-          ptx::bulk_g2s(ring + (size_t)st * tile_bytes, reinterpret_cast<const void*>(p.h2d ? a.cpu : a.gpu),
-                        a.bytes, &full[st]);
-        }
-      }
+      desc[(base + lane) & (kDescRing - 1)] = d;
       major += step_q;
       r += step_r;
       if (r >= span) { r -= span; ++major; }
+      fetch(base + 32 + lane);
     }
+    __syncwarp();
+    if (lane == 0) {
+      const int32_t end = min(base + 32, n_steps);
+      for (int32_t it = base; it < end; ++it) {
+        const int32_t j = it - LOOKAHEAD;
+        if (j >= 0) {
+          const TileDesc& d = desc[j & (kDescRing - 1)];
+          if (signalling && d.major > signalled) {
+            // first store of a later layer: everything this warp owned in the earlier layers is committed;
+            // drain those stores (the loads in flight are unaffected) and post the layers
+            ptx::bulk_wait<0>();
+            __threadfence_block();
+            *reinterpret_cast<volatile int*>(&s_layers_done[warp]) = d.major;
+            signalled = d.major;
+          }
+          if (d.bytes) {
+            if (!ptx::mbar_wait_bounded(&full[st_st], (phases >> st_st) & 1u, kWaitBudgetNs)) {
+              dead = 1;
+              break;
+            }
+            phases ^= 1u << st_st;
+            ptx::bulk_s2g(reinterpret_cast<void*>(d.dst), ring + (size_t)st_st * tile_bytes, d.bytes);
+          }
+          ptx::bulk_commit();  // one group per tile (possibly empty) keeps the wait arithmetic uniform
+          if (++st_st == STAGES) st_st = 0;
+        }
+        if (it < n_mine) {
+          const TileDesc& d = desc[it & (kDescRing - 1)];
+          // the stage was last used by tile it-STAGES; all but the newest
+          // STAGES-LOOKAHEAD store groups must have finished reading smem
+          if (it >= STAGES) ptx::bulk_wait_read<STAGES - LOOKAHEAD>();
+          if (d.bytes) {
+            ptx::mbar_expect_tx(&full[ld_st], d.bytes);
+            ptx::bulk_g2s(ring + (size_t)ld_st * tile_bytes, reinterpret_cast<const void*>(d.src), d.bytes,
+                          &full[ld_st]);
+          }
+          if (++ld_st == STAGES) ld_st = 0;
+        }
+      }
+    }
+    dead = __shfl_sync(0xffffffffu, dead, 0);   // also orders lane 0's reads before the next batch is written
+    if (dead) break;
   }
+  err = (int)__reduce_or_sync(0xffffffffu, (unsigned)err);
   if (lane == 0) {
+    if (dead) err |= KV_ERR_WAIT_EXPIRED;
     ptx::bulk_wait<0>();
     if (err && p.status) report_status(p.status, err);
     if (p.layer_major) {
-      if (has_signaller) {
-        __threadfence_block();
-        *reinterpret_cast<volatile int*>(&s_layers_done) = p.num_layers;   // every exit path ends here
-      } else {
-        signal_layers(p, signalled, p.num_layers);
-      }
+      __threadfence_block();
+      *reinterpret_cast<volatile int*>(&s_layers_done[warp]) = p.num_layers;   // every exit path ends here
     } else {
-      signal_done(p);
+      signal_done(p, gridDim.x * W);
     }
   }
 }
@@ -316,14 +330,14 @@ cudaError_t ensure_smem(K kernel, int bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-template <int STAGES, int LA>
+template <int W, int STAGES, int LA>
 cudaError_t launch_bulk(const KvCopyParams& p, int ctas, int tile_bytes, int tiles_per_chunk, cudaStream_t s) {
-  const int smem = STAGES * tile_bytes;
-  auto k = kv_copy_bulk_kernel<STAGES, LA>;
+  const int smem = W * STAGES * tile_bytes;
+  auto k = kv_copy_bulk_kernel<W, STAGES, LA>;
   cudaError_t e = ensure_smem(k, smem);
   if (e != cudaSuccess) return e;
-  const int threads = (p.layer_major && p.done_counter != nullptr) ? 64 : 32;   // second warp = layer signaller
-  k<<<ctas, threads, smem, s>>>(p, tile_bytes, tiles_per_chunk);
+  const int warps = W + (p.layer_major && p.done_counter != nullptr ? 1 : 0);   // last warp = layer signaller
+  k<<<ctas, 32 * warps, smem, s>>>(p, tile_bytes, tiles_per_chunk);
   return cudaGetLastError();
 }
 
@@ -364,21 +378,19 @@ cudaError_t launch_kv_copy(const KvCopyParams& p, const KvCopyLaunch& cfg, cudaS
     const int64_t total = (int64_t)p.num_pairs * p.num_layers * p.kv_dim * tiles_per_chunk;
     int ctas = cfg.num_ctas > 0 ? cfg.num_ctas : 16;
     if ((int64_t)ctas > total) ctas = (int)total;
-    // deepest ring that fits beside the static barriers (limit 227 KiB per CTA)
-    const int budget = 200 * 1024;
-    const int stages = budget / tile;
+    // Pipelines per CTA and the depth of their rings: together they hold at most 192 KiB of the 227 KiB a CTA may
+    // have, whatever the tile. Host reads need bytes in flight to cover the PCIe round trip, so host->GPU keeps
+    // every stage but one loading; GPU->host leaves half of a deep ring to queued posted writes.
     if (p.h2d) {
-      if (stages >= 32) return launch_bulk<32, 31>(p, ctas, tile, tiles_per_chunk, stream);
-      if (stages >= 20) return launch_bulk<20, 19>(p, ctas, tile, tiles_per_chunk, stream);
-      if (stages >= 12) return launch_bulk<12, 11>(p, ctas, tile, tiles_per_chunk, stream);
-      if (stages >= 8) return launch_bulk<8, 7>(p, ctas, tile, tiles_per_chunk, stream);
-      return launch_bulk<6, 5>(p, ctas, tile, tiles_per_chunk, stream);
+      if (tile <= 4096) return launch_bulk<4, 12, 11>(p, ctas, tile, tiles_per_chunk, stream);
+      if (tile <= 8192) return launch_bulk<4, 6, 5>(p, ctas, tile, tiles_per_chunk, stream);
+      if (tile <= 16384) return launch_bulk<4, 3, 2>(p, ctas, tile, tiles_per_chunk, stream);
+      return launch_bulk<2, 3, 2>(p, ctas, tile, tiles_per_chunk, stream);
     }
-    if (stages >= 32) return launch_bulk<32, 16>(p, ctas, tile, tiles_per_chunk, stream);
-    if (stages >= 20) return launch_bulk<20, 10>(p, ctas, tile, tiles_per_chunk, stream);
-    if (stages >= 12) return launch_bulk<12, 6>(p, ctas, tile, tiles_per_chunk, stream);
-    if (stages >= 8) return launch_bulk<8, 4>(p, ctas, tile, tiles_per_chunk, stream);
-    return launch_bulk<6, 3>(p, ctas, tile, tiles_per_chunk, stream);
+    if (tile <= 4096) return launch_bulk<4, 12, 6>(p, ctas, tile, tiles_per_chunk, stream);
+    if (tile <= 8192) return launch_bulk<4, 6, 3>(p, ctas, tile, tiles_per_chunk, stream);
+    if (tile <= 16384) return launch_bulk<4, 3, 2>(p, ctas, tile, tiles_per_chunk, stream);
+    return launch_bulk<2, 3, 2>(p, ctas, tile, tiles_per_chunk, stream);
   }
   // SIMT engine
   if (tile > p.chunk_bytes) tile = (int)p.chunk_bytes;

@@ -172,3 +172,34 @@ def test_large_transfer_exceeds_l2_and_is_exact():
     gi = torch.from_numpy(g).to(dev)
     for l in range(shape.num_layers):
         assert torch.equal(tensors[l][:, gi], saved[l][:, gi])
+
+
+@pytest.mark.parametrize("chunk", [16, 256, 1008, 4096, 4112, 8208, 16384, 16400, 65552])
+@pytest.mark.parametrize("n,ctas", [(1, 8), (5, 1), (67, 3)])
+def test_bulk_engine_at_tile_and_batch_edges(chunk, n, ctas):
+    """Chunks around the tile sizes at which ring depth and pipelines per CTA change, op sizes from fewer tiles than
+    pipelines to several 32-tile descriptor batches with a remainder, both directions; bytes are exact."""
+    dev = torch.device("cuda:0")
+    shape = KVShape("edge", 3, 1, chunk, dtype=torch.uint8, use_mla=True, tokens_per_block=1)
+    NB = n + 4
+    rng = np.random.default_rng(chunk + n)
+    for tile in (1024, 16384, 32768):
+        tensors, layout = alloc_paged_cache(shape, NB, dev, "vllm", fill="normal", seed=tile)
+        reg = register_tensors(tensors, layout)
+        pool, side, _ = _host_pool(shape, NB)
+        g = rng.permutation(NB)[:n].astype(np.int64)
+        c = rng.permutation(NB)[:n].astype(np.int64)
+        status = new_status(dev)
+        keep = kv_copy(reg, side, g, c, h2d=False, num_ctas=ctas, tile_bytes=tile, status=status)
+        torch.cuda.synchronize()
+        want = torch.stack([t.view(NB, -1) for t in tensors], 1)[torch.from_numpy(g).to(dev)]
+        assert torch.equal(pool[torch.from_numpy(c)].view(n, 3, -1), want.cpu())
+        for t in tensors:
+            t.zero_()
+        keep += kv_copy(reg, side, g, c, h2d=True, num_ctas=ctas, tile_bytes=tile, status=status)
+        torch.cuda.synchronize()
+        got = torch.stack([t.view(NB, -1) for t in tensors], 1)
+        assert decode_status(status) == 0 and torch.equal(got[torch.from_numpy(g).to(dev)], want)
+        rest = torch.ones(NB, dtype=torch.bool)
+        rest[torch.from_numpy(g)] = False
+        assert int(got[rest.to(dev)].abs().sum()) == 0
