@@ -178,6 +178,20 @@ void init_kernel_bindings(py::module_& m) {
   }, py::arg("tokens"), py::arg("offsets"), py::arg("num_seqs"), py::arg("tokens_per_block"), py::arg("ns_prefix") = 0,
      py::arg("ns_len") = 0, py::arg("out") = 0, py::arg("out_offsets") = 0, py::arg("stream") = 0);
 
+  // The same for a list of sequences anywhere on the device; `ns` holds the prefix values as bytes.
+  m.def("kv_block_hashes_list", [](const std::vector<uint64_t>& tokens, const std::vector<int64_t>& lens,
+                                   int tokens_per_block, const std::string& ns, uint64_t out, uint64_t stream) {
+    if (tokens.size() != lens.size() || tokens.size() > (size_t)kHashListSeqs || ns.size() > (size_t)kHashListNs)
+      throw std::invalid_argument("kv_block_hashes_list: too many sequences or prefix values");
+    throw_on(launch_kv_block_hashes_list(reinterpret_cast<const int64_t* const*>(tokens.data()), lens.data(),
+                                         (int)tokens.size(), tokens_per_block, (const uint8_t*)ns.data(),
+                                         (int)ns.size(), (uint64_t*)(uintptr_t)out, (cudaStream_t)(uintptr_t)stream),
+             "kv_block_hashes launch");
+  }, py::arg("tokens"), py::arg("lens"), py::arg("tokens_per_block"), py::arg("ns") = py::bytes(), py::arg("out") = 0,
+     py::arg("stream") = 0);
+  m.attr("HASH_LIST_SEQS") = kHashListSeqs;
+  m.attr("HASH_LIST_NS") = kHashListNs;
+
   m.def("host_kv_copy", [](py::dict params, int threads) {
     KvCopyParams p = kv_params_from_dict(params, true);
     py::gil_scoped_release rel;

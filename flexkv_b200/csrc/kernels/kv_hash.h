@@ -12,9 +12,19 @@ namespace fkv {
 
 // tokens: all sequences back to back; offsets[n+1] (in tokens) and out_offsets[n+1] (in blocks)
 // are device- or mapped-host-readable. ns_prefix (ns_len int64 values, may be null) is fed
-// before every sequence. One quad of threads hashes one sequence.
+// before every sequence.
 cudaError_t launch_kv_block_hashes(const int64_t* tokens, const int64_t* offsets, int64_t num_seqs, int tokens_per_block,
                                    const int64_t* ns_prefix, int64_t ns_len, uint64_t* out, const int64_t* out_offsets,
                                    cudaStream_t stream);
+
+constexpr int kHashListSeqs = 128;   // sequences whose addresses travel in the launch parameters
+constexpr int kHashListNs = 256;     // namespace bytes that do
+
+// The same for at most kHashListSeqs sequences that lie anywhere on the device: no concatenation and no offset
+// tables to upload. tokens[i] / lens[i]: device address and length of sequence i (lengths below 2^31); the keys of
+// sequence i follow those of sequence i-1 in `out`. ns: at most kHashListNs prefix values, each one byte.
+cudaError_t launch_kv_block_hashes_list(const int64_t* const* tokens, const int64_t* lens, int num_seqs,
+                                        int tokens_per_block, const uint8_t* ns, int ns_len, uint64_t* out,
+                                        cudaStream_t stream);
 
 }  // namespace fkv

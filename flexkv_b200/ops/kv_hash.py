@@ -19,22 +19,34 @@ def gpu_block_hashes(seqs: Sequence[torch.Tensor], tokens_per_block: int, namesp
     if not seqs:
         return []
     dev = seqs[0].device
-    lens = [int(s.numel()) for s in seqs]
-    flat = torch.cat([s.reshape(-1) for s in seqs]) if len(seqs) > 1 else seqs[0].reshape(-1).contiguous()
-    offs = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int64, device=dev)
-    nblk = [n // tokens_per_block for n in lens]
-    ooffs = torch.tensor(np.concatenate([[0], np.cumsum(nblk)]), dtype=torch.int64, device=dev)
-    out = torch.empty(max(1, sum(nblk)), dtype=torch.int64, device=dev)
-    ns = namespace_prefix(namespace)
-    ns_t = torch.from_numpy(np.ascontiguousarray(ns, dtype=np.int64)).to(dev) if ns is not None and len(ns) else None
+    C = _native.C
     s = stream if stream is not None else torch.cuda.current_stream(dev)
-    _native.C.kv_block_hashes(flat.data_ptr(), offs.data_ptr(), len(seqs), int(tokens_per_block),
-                              ns_t.data_ptr() if ns_t is not None else 0, int(ns_t.numel()) if ns_t is not None else 0,
-                              out.data_ptr(), ooffs.data_ptr(), s.cuda_stream)
-    res, o = [], 0
-    for n in nblk:
-        res.append(out[o:o + n])
-        o += n
-    # keep inputs alive until the launch has been ordered on the stream
-    flat.record_stream(s)
-    return res
+    lens = [t.numel() for t in seqs]
+    nblk = [n // tokens_per_block for n in lens]
+    ns = namespace_prefix(namespace)
+    out = torch.empty(sum(nblk), dtype=torch.int64, device=dev)
+    side = s != torch.cuda.current_stream(dev)
+    if side:
+        s.wait_stream(torch.cuda.current_stream(dev))
+    if len(seqs) <= C.HASH_LIST_SEQS and (ns is None or ns.size <= C.HASH_LIST_NS) and max(lens) < 2**31:
+        # the sequences stay where they are: addresses, lengths and prefix travel in the launch parameters
+        seqs = [t if t.dtype == torch.int64 and t.is_contiguous() else t.to(torch.int64).contiguous() for t in seqs]
+        C.kv_block_hashes_list([t.data_ptr() for t in seqs], lens, int(tokens_per_block),
+                               b"" if ns is None else ns.astype(np.uint8).tobytes(), out.data_ptr(), s.cuda_stream)
+        if side:
+            for t in seqs + [out]:
+                t.record_stream(s)
+        return list(out.split(nblk))
+    flat = torch.cat([t.reshape(-1) for t in seqs]).to(torch.int64)
+    offs = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int64, device=dev)
+    ooffs = torch.tensor(np.concatenate([[0], np.cumsum(nblk)]), dtype=torch.int64, device=dev)
+    ns_t = torch.from_numpy(np.ascontiguousarray(ns, dtype=np.int64)).to(dev) if ns is not None and len(ns) else None
+    C.kv_block_hashes(flat.data_ptr(), offs.data_ptr(), len(seqs), int(tokens_per_block),
+                      ns_t.data_ptr() if ns_t is not None else 0, int(ns_t.numel()) if ns_t is not None else 0,
+                      out.data_ptr(), ooffs.data_ptr(), s.cuda_stream)
+    if side:
+        # the temporaries and the keys stay alive until the stream has passed the launch
+        for t in (flat, offs, ooffs, ns_t, out):
+            if t is not None:
+                t.record_stream(s)
+    return list(out.split(nblk))

@@ -33,3 +33,19 @@ def test_large_batch_is_consistent():
     torch.cuda.synchronize()
     for i in (0, 1, 150, 299):
         assert got[i].cpu().numpy().view(np.uint64).tolist() == hash_blocks(seqs[i], 16).tolist()
+
+
+@pytest.mark.parametrize("nseq,lens", [(3, (1024, 1025, 1023)), (128, (2047, 2048, 2050)), (129, (1027, 3)),
+                                       (900, (129, 127, 4100))])
+@pytest.mark.parametrize("tpb,namespace", [(1, None), (16, ["x"]), (64, ["tenant" * 50])])
+def test_segment_edges_and_both_forms(nseq, lens, tpb, namespace):
+    """Lengths around the segment size of either kernel form (one and eight sequences per CTA), sequence counts on
+    both sides of the list form's limit and of the change of form, prefixes on both sides of the inline limit; an
+    empty sequence among them, and a stream of its own."""
+    dev = torch.device("cuda:0")
+    rng = np.random.default_rng(nseq + tpb)
+    seqs = [rng.integers(-2**62, 2**62, size=lens[i % len(lens)] if i != 1 else 0, dtype=np.int64) for i in range(nseq)]
+    got = gpu_block_hashes([torch.from_numpy(s).to(dev) for s in seqs], tpb, namespace, stream=torch.cuda.Stream(dev))
+    torch.cuda.synchronize()
+    for i in sorted({0, 1, 2, nseq // 2, nseq - 2, nseq - 1}):
+        assert got[i].cpu().numpy().view(np.uint64).tolist() == hash_blocks(seqs[i], tpb, namespace).tolist()
