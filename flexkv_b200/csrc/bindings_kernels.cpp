@@ -219,6 +219,24 @@ void init_kernel_bindings(py::module_& m) {
     return py::make_tuple(runs, std::string(names[(int)path]), ce_num_copies(a, p, path), a.status);
   }, py::arg("params"), py::arg("max_copies") = 4096, py::arg("min_bytes_per_copy") = 8 << 20);
 
+  // Plan of the staged route: (pieces [P, 3] of first pair, host block, length; pairs staged; gpu ids and host ids as
+  // reordered), or None when the op stays with the kernel.
+  m.def("ce_stage_plan", [](py::dict params, int64_t min_run, int64_t max_piece) -> py::object {
+    KvCopyParams p = kv_params_from_dict(params, true);
+    std::vector<int64_t> g(p.gpu_blocks, p.gpu_blocks + p.num_pairs), c(p.cpu_blocks, p.cpu_blocks + p.num_pairs);
+    CeStagePlan plan;
+    if (!ce_plan_staged(p, g.data(), c.data(), min_run, max_piece, plan)) return py::none();
+    py::array_t<int64_t> pieces(std::vector<py::ssize_t>{(py::ssize_t)plan.pieces.size(), 3});
+    auto r = pieces.mutable_unchecked<2>();
+    for (size_t i = 0; i < plan.pieces.size(); ++i) {
+      r(i, 0) = plan.pieces[i].first;
+      r(i, 1) = plan.pieces[i].cpu_block;
+      r(i, 2) = plan.pieces[i].len;
+    }
+    return py::make_tuple(pieces, plan.staged, py::array_t<int64_t>((py::ssize_t)g.size(), g.data()),
+                          py::array_t<int64_t>((py::ssize_t)c.size(), c.data()));
+  }, py::arg("params"), py::arg("min_run"), py::arg("max_piece"));
+
   m.def("kv_copy_tma_eligible", [](py::dict params) { return kv_copy_tma_eligible(kv_params_from_dict(params, true)); });
   m.def("ptr_table_cache_size", &ptr_table_cache_size);
   m.attr("MAX_GPU_PTRS_EXT") = kMaxGpuPtrsExt;

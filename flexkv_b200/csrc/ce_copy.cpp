@@ -107,12 +107,13 @@ cudaError_t ce_copy(const KvCopyParams& p, const CeAnalysis& a, CePath path, cud
 // ---------------------------------------------------------------- staged route
 
 void ce_staging_free(CeStaging& st) {
-  for (int b = 0; b < 2; ++b) {
+  for (int b = 0; b < kCeStageBufs; ++b) {
     if (st.buf[b]) cudaFree(st.buf[b]);
     if (st.kernel_done[b]) cudaEventDestroy(st.kernel_done[b]);
     if (st.copy_done[b]) cudaEventDestroy(st.copy_done[b]);
     st.buf[b] = nullptr;
     st.kernel_done[b] = st.copy_done[b] = nullptr;
+    st.used[b] = false;
   }
   if (st.iota) cudaFree(st.iota);
   if (st.copy_stream) cudaStreamDestroy(st.copy_stream);
@@ -121,31 +122,14 @@ void ce_staging_free(CeStaging& st) {
   st.blocks = 0;
 }
 
-bool ce_host_runs(const KvCopyParams& p, const int64_t* g, const int64_t* c, int64_t n, int total_layers,
-                  int64_t min_run, std::vector<CeHostRun>& runs) {
-  runs.clear();
-  if (n <= 0 || p.c_use_table || p.layer_start != 0 || p.num_layers != total_layers || p.c_off != 0) return false;
-  if (p.c_kv_stride != p.chunk_bytes || p.c_layer_stride != p.chunk_bytes * p.kv_dim ||
-      p.c_block_stride != p.c_layer_stride * p.num_layers)
-    return false;                                          // host blocks do not abut in [layer][kv][chunk] order
-  for (int64_t i = 0; i < n; ++i) {
-    if (p.gpu_num_blocks > 0 && (g[i] < 0 || g[i] >= p.gpu_num_blocks)) return false;
-    if (p.cpu_num_blocks > 0 && (c[i] < 0 || c[i] >= p.cpu_num_blocks)) return false;
-    if (!runs.empty() && c[i] == runs.back().cpu_block + runs.back().len) {
-      ++runs.back().len;
-      continue;
-    }
-    if (!runs.empty() && runs.back().len < min_run) return false;
-    runs.push_back(CeHostRun{i, c[i], 1});
-  }
-  return runs.back().len >= min_run;
-}
-
-static cudaError_t staging_prepare(CeStaging& st, int64_t blocks, int64_t block_bytes) {
-  if (st.blocks >= blocks && st.block_bytes == block_bytes) return cudaSuccess;
+bool ce_staging_prepare(CeStaging& st, int64_t blocks, int64_t block_bytes) {
+  if (block_bytes <= 0) return false;
+  if (blocks <= 0) blocks = std::max<int64_t>(1, kCeStageBytes / block_bytes);
+  if (st.blocks >= blocks && st.block_bytes == block_bytes) return true;
+  if (st.refused) return false;
   ce_staging_free(st);
   cudaError_t e = cudaSuccess;
-  for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
+  for (int b = 0; b < kCeStageBufs && e == cudaSuccess; ++b) {
     e = cudaMalloc((void**)&st.buf[b], (size_t)(blocks * block_bytes));
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&st.kernel_done[b], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&st.copy_done[b], cudaEventDisableTiming);
@@ -158,60 +142,128 @@ static cudaError_t staging_prepare(CeStaging& st, int64_t blocks, int64_t block_
   }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st.copy_stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
+    (void)cudaGetLastError();
     ce_staging_free(st);
-    return e;
+    st.refused = true;
+    return false;
   }
   st.blocks = blocks;
   st.block_bytes = block_bytes;
-  st.used[0] = st.used[1] = false;
-  return cudaSuccess;
+  return true;
 }
 
-cudaError_t ce_copy_staged(const KvCopyParams& p, const std::vector<CeHostRun>& runs, CeStaging& st,
-                           int64_t staging_blocks, const KvCopyLaunch& cfg, cudaStream_t stream) {
-  const int64_t block_bytes = p.c_block_stride;
-  cudaError_t e = staging_prepare(st, staging_blocks, block_bytes);
-  if (e != cudaSuccess) return e;
-  int k = 0;
-  for (const CeHostRun& r : runs) {
-    for (int64_t lo = 0; lo < r.len; lo += st.blocks, ++k) {
-      const int b = k & 1;
-      const int64_t m = std::min(st.blocks, r.len - lo);
-      uint8_t* host = reinterpret_cast<uint8_t*>(p.cpu_base) + (r.cpu_block + lo) * block_bytes;
-      KvCopyParams q = p;            // the staging buffer plays the host side, in host block format
-      q.cpu_base = reinterpret_cast<uint64_t>(st.buf[b]);
-      q.gpu_blocks = p.gpu_blocks + r.first + lo;
-      q.cpu_blocks = st.iota;
-      q.num_pairs = (int32_t)m;
-      q.cpu_num_blocks = st.blocks;
-      q.done_counter = nullptr;
-      q.dev_flags = q.host_flags = nullptr;
-      q.layer_major = 0;
-      if (!p.h2d) {
-        // gather on `stream` once the previous copy out of this buffer is done, then one large copy
-        if (st.used[b]) e = cudaStreamWaitEvent(stream, st.copy_done[b], 0);
-        if (e == cudaSuccess) e = launch_kv_copy(q, cfg, stream);
-        if (e == cudaSuccess) e = cudaEventRecord(st.kernel_done[b], stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(st.copy_stream, st.kernel_done[b], 0);
-        if (e == cudaSuccess)
-          e = cudaMemcpyAsync(host, st.buf[b], (size_t)(m * block_bytes), cudaMemcpyDeviceToHost, st.copy_stream);
-        if (e == cudaSuccess) e = cudaEventRecord(st.copy_done[b], st.copy_stream);
-      } else {
-        // one large copy in once the previous scatter out of this buffer is done, then the scatter kernel
-        if (st.used[b]) e = cudaStreamWaitEvent(st.copy_stream, st.kernel_done[b], 0);
-        if (e == cudaSuccess)
-          e = cudaMemcpyAsync(st.buf[b], host, (size_t)(m * block_bytes), cudaMemcpyHostToDevice, st.copy_stream);
-        if (e == cudaSuccess) e = cudaEventRecord(st.copy_done[b], st.copy_stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, st.copy_done[b], 0);
-        if (e == cudaSuccess) e = launch_kv_copy(q, cfg, stream);
-        if (e == cudaSuccess) e = cudaEventRecord(st.kernel_done[b], stream);
-      }
-      if (e != cudaSuccess) return e;
-      st.used[b] = true;
-    }
+bool ce_host_blocks_abut(const KvCopyParams& p, int total_layers, int64_t chunk_slot) {
+  return !p.c_use_table && p.layer_start == 0 && p.num_layers == total_layers && p.num_layers > 0 && p.kv_dim > 0 &&
+         chunk_slot > 0 && p.c_off == 0 && p.c_kv_stride == chunk_slot && p.c_layer_stride == chunk_slot * p.kv_dim &&
+         p.c_block_stride == p.c_layer_stride * p.num_layers;
+}
+
+bool ce_plan_staged(const KvCopyParams& p, int64_t* g, int64_t* c, int64_t min_run, int64_t max_piece,
+                    CeStagePlan& plan) {
+  plan.pieces.clear();
+  plan.staged = 0;
+  const int64_t n = p.num_pairs;
+  if (n <= 0 || max_piece <= 0 || p.c_block_stride <= 0) return false;
+  std::vector<CeHostRun> runs;
+  for (int64_t i = 0; i < n; ++i) {
+    if (p.gpu_num_blocks > 0 && (g[i] < 0 || g[i] >= p.gpu_num_blocks)) return false;
+    if (p.cpu_num_blocks > 0 && (c[i] < 0 || c[i] >= p.cpu_num_blocks)) return false;
+    if (!runs.empty() && c[i] == runs.back().cpu_block + runs.back().len) ++runs.back().len;
+    else runs.push_back(CeHostRun{i, c[i], 1});
   }
+  int64_t staged = 0;
+  for (const CeHostRun& r : runs)
+    if (r.len >= min_run) staged += r.len;
+  if (staged == 0) return false;
+  if (staged < n) {
+    if (staged * p.c_block_stride < kCeMixedMinBytes) return false;
+    std::vector<int64_t> g2, c2;
+    g2.reserve((size_t)n);
+    c2.reserve((size_t)n);
+    for (int part = 0; part < 2; ++part)
+      for (CeHostRun& r : runs) {
+        if ((r.len >= min_run) != (part == 0)) continue;
+        const int64_t at = (int64_t)g2.size();
+        g2.insert(g2.end(), g + r.first, g + r.first + r.len);
+        c2.insert(c2.end(), c + r.first, c + r.first + r.len);
+        r.first = at;
+      }
+    std::copy(g2.begin(), g2.end(), g);
+    std::copy(c2.begin(), c2.end(), c);
+  }
+  // small pieces where the kernel has the link to itself: first in an offload, last in a restore
+  int64_t next = std::min(max_piece, std::max<int64_t>(1, kCeRampBytes / p.c_block_stride));
+  auto cut = [&](const CeHostRun& r) {
+    for (int64_t done = 0; done < r.len;) {
+      const int64_t m = std::min(next, r.len - done);
+      const int64_t at = p.h2d ? r.len - done - m : done;
+      plan.pieces.push_back(CeHostRun{r.first + at, r.cpu_block + at, m});
+      done += m;
+      next = std::min(max_piece, next * 2);
+    }
+  };
+  if (p.h2d) {
+    for (size_t i = runs.size(); i-- > 0;)
+      if (runs[i].len >= min_run) cut(runs[i]);
+    std::reverse(plan.pieces.begin(), plan.pieces.end());
+  } else {
+    for (const CeHostRun& r : runs)
+      if (r.len >= min_run) cut(r);
+  }
+  plan.staged = staged;
+  return true;
+}
+
+cudaError_t ce_copy_staged(const KvCopyParams& p, const CeStagePlan& plan, CeStaging& st, const CeStageKernel& kernel,
+                           cudaStream_t stream) {
+  const int64_t block_bytes = p.c_block_stride;
+  cudaError_t e = cudaSuccess;
+  auto others = [&]() -> cudaError_t {
+    if (plan.staged >= p.num_pairs) return cudaSuccess;
+    KvCopyParams q = p;
+    q.gpu_blocks = p.gpu_blocks + plan.staged;
+    q.cpu_blocks = p.cpu_blocks + plan.staged;
+    q.num_pairs = (int32_t)(p.num_pairs - plan.staged);
+    return kernel(q, 0, stream);
+  };
+  if (p.h2d) e = others();
+  int b = 0;
+  for (const CeHostRun& piece : plan.pieces) {
+    if (e != cudaSuccess) return e;
+    uint8_t* host = reinterpret_cast<uint8_t*>(p.cpu_base) + piece.cpu_block * block_bytes;
+    const size_t bytes = (size_t)(piece.len * block_bytes);
+    KvCopyParams q = p;            // the staging buffer plays the host side, in host block format
+    q.cpu_base = reinterpret_cast<uint64_t>(st.buf[b]);
+    q.gpu_blocks = p.gpu_blocks + piece.first;
+    q.cpu_blocks = st.iota;
+    q.num_pairs = (int32_t)piece.len;
+    q.cpu_num_blocks = st.blocks;
+    q.done_counter = nullptr;
+    q.dev_flags = q.host_flags = nullptr;
+    q.layer_major = 0;
+    if (!p.h2d) {
+      // gather on `stream` once the previous copy out of this buffer is done, then one large copy
+      if (st.used[b]) e = cudaStreamWaitEvent(stream, st.copy_done[b], 0);
+      if (e == cudaSuccess) e = kernel(q, piece.cpu_block, stream);
+      if (e == cudaSuccess) e = cudaEventRecord(st.kernel_done[b], stream);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st.copy_stream, st.kernel_done[b], 0);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(host, st.buf[b], bytes, cudaMemcpyDeviceToHost, st.copy_stream);
+      if (e == cudaSuccess) e = cudaEventRecord(st.copy_done[b], st.copy_stream);
+    } else {
+      // one large copy in once the previous scatter out of this buffer is done, then the scatter kernel
+      if (st.used[b]) e = cudaStreamWaitEvent(st.copy_stream, st.kernel_done[b], 0);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(st.buf[b], host, bytes, cudaMemcpyHostToDevice, st.copy_stream);
+      if (e == cudaSuccess) e = cudaEventRecord(st.copy_done[b], st.copy_stream);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, st.copy_done[b], 0);
+      if (e == cudaSuccess) e = kernel(q, piece.cpu_block, stream);
+      if (e == cudaSuccess) e = cudaEventRecord(st.kernel_done[b], stream);
+    }
+    if (e == cudaSuccess) st.used[b] = true;
+    b = b + 1 == kCeStageBufs ? 0 : b + 1;
+  }
+  if (!p.h2d && e == cudaSuccess) e = others();
   // the caller's stream ends after the last copies
-  for (int b = 0; b < 2 && e == cudaSuccess; ++b)
+  for (b = 0; b < kCeStageBufs && e == cudaSuccess; ++b)
     if (st.used[b]) e = cudaStreamWaitEvent(stream, st.copy_done[b], 0);
   return e;
 }

@@ -16,6 +16,7 @@
 // streams, below the kernel's 52.8 / 51.5, and a host-side scatter would spend CPU cores and memory bandwidth.
 #pragma once
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -59,32 +60,66 @@ int64_t ce_num_copies(const CeAnalysis& a, const KvCopyParams& p, CePath path);
 cudaError_t ce_copy(const KvCopyParams& p, const CeAnalysis& a, CePath path, cudaStream_t stream);
 
 // ---- staged route -------------------------------------------------------------------------------------------
+// A run of consecutive host blocks over consecutive pairs of the op.
 struct CeHostRun {
   int64_t first;      // index of the run's first pair in the op's id arrays
   int64_t cpu_block;  // its first host block
   int64_t len;
 };
 
-// Device staging of one GPU (owned by the caller's per-rank state; allocated on first use, freed by ce_staging_free).
+// How an op is split: pairs [0, staged) cross the link in pieces, one large copy each; the others, whose host
+// blocks stand alone, stay with the kernel.
+struct CeStagePlan {
+  std::vector<CeHostRun> pieces;   // in the order they are moved; none longer than a staging buffer
+  int64_t staged = 0;
+};
+
+constexpr int kCeStageBufs = 2;
+// Bytes of one staging buffer unless a caller asks for a number of blocks. B200, contiguous copies back to back,
+// GB/s GPU->host / host->GPU: pieces of 4 MiB 54.1 / 52.5, 16 MiB 56.2 / 54.8, 64 MiB 56.6 / 55.4, one of 1 GiB
+// 57.0 / 55.6.
+constexpr int64_t kCeStageBytes = 32 << 20;
+// An op moves kernel-first until its first piece is gathered (and kernel-last for a restore), so that piece is small
+// and the following ones double.
+constexpr int64_t kCeRampBytes = 4 << 20;
+// Bytes that the runs must hold before an op is split between copy engine and kernel: about 8 % of their time is
+// won, and the second launch and the events cost some 20 us.
+constexpr int64_t kCeMixedMinBytes = 32 << 20;
+
+// Device staging of one GPU (owned by the caller's per-rank state, freed by ce_staging_free).
 struct CeStaging {
-  uint8_t* buf[2] = {nullptr, nullptr};
+  uint8_t* buf[kCeStageBufs] = {};
   int64_t* iota = nullptr;            // device array 0, 1, 2, ...: the staged block ids
-  cudaEvent_t kernel_done[2] = {nullptr, nullptr}, copy_done[2] = {nullptr, nullptr};
+  cudaEvent_t kernel_done[kCeStageBufs] = {}, copy_done[kCeStageBufs] = {};
   cudaStream_t copy_stream = nullptr;
   int64_t blocks = 0, block_bytes = 0;
-  bool used[2] = {false, false};
+  bool used[kCeStageBufs] = {};
+  bool refused = false;               // there was no memory for it: not asked for again
 };
+// Makes room for `blocks` blocks per buffer (0: kCeStageBytes' worth) on the current device. False when the
+// device has no memory for it; the op then stays with the kernel.
+bool ce_staging_prepare(CeStaging& st, int64_t blocks, int64_t block_bytes);
 void ce_staging_free(CeStaging& st);
 
-// Maximal runs of consecutive host block ids over consecutive pairs. Returns false (and leaves `runs` unspecified)
-// unless every pair lies in a run of at least `min_run` blocks, all ids are in range, the op covers whole host
-// blocks (layer_start == 0, every layer) and consecutive host blocks abut in memory in [layer][kv][chunk] order.
-bool ce_host_runs(const KvCopyParams& p, const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n,
-                  int total_layers, int64_t min_run, std::vector<CeHostRun>& runs);
-// Moves the op through the staging area: pieces of at most `staging_blocks` blocks, gather/scatter kernel on
-// `stream`, large copies on the staging's own stream, two buffers in flight. When it returns, everything has
-// been queued and `stream` waits for the last copy.
-cudaError_t ce_copy_staged(const KvCopyParams& p, const std::vector<CeHostRun>& runs, CeStaging& st,
-                           int64_t staging_blocks, const KvCopyLaunch& cfg, cudaStream_t stream);
+// True when the host side of `p` is whole blocks of [layer][kv][chunk_slot] that abut, so that consecutive block ids
+// are one span of memory.
+bool ce_host_blocks_abut(const KvCopyParams& p, int total_layers, int64_t chunk_slot);
+
+// Plans the staged route for an op whose host blocks abut. Runs of at least `min_run` consecutive host blocks become
+// pieces of at most `max_piece` blocks; where they leave other pairs over, the id arrays are REORDERED in place (runs
+// first) and the op is only split when the runs hold at least kCeMixedMinBytes. False, with the arrays as they were,
+// when the op belongs to the kernel: an id out of range, no run long enough.
+bool ce_plan_staged(const KvCopyParams& p, int64_t* gpu_blocks, int64_t* cpu_blocks, int64_t min_run,
+                    int64_t max_piece, CeStagePlan& plan);
+
+// Launches the kernel of a piece or of the pairs that stay with it. For a piece, `q` addresses the staging buffer as
+// the host side (block ids 0, 1, ...) and `host_block` is the host block that id 0 stands for; otherwise it is 0.
+using CeStageKernel = std::function<cudaError_t(const KvCopyParams& q, int64_t host_block, cudaStream_t stream)>;
+// Moves the op: pieces through the staging buffers, gather or scatter kernel on `stream`, large copies on the
+// staging's own stream, both buffers in flight; the other pairs by the kernel, on `stream`, beside the last copies
+// (offload) or the first ones (restore). When it returns, everything has been queued and `stream` waits for the last
+// copy. `p` carries the id arrays as planned.
+cudaError_t ce_copy_staged(const KvCopyParams& p, const CeStagePlan& plan, CeStaging& st, const CeStageKernel& kernel,
+                           cudaStream_t stream);
 
 }  // namespace fkv

@@ -324,20 +324,23 @@ __global__ void __launch_bounds__(1024) kv_copy_refshape_kernel(const __grid_con
   }
 }
 
-template <typename K>
-cudaError_t ensure_smem(K kernel, int bytes) {
+// Dynamic shared memory that every instance may ask for: its rings at the largest tile it serves. One figure for
+// all, so that threads launching ops of different tile sizes cannot lower it under one another.
+constexpr int kRingBytes = 192 << 10;
+
+template <int W, int STAGES, int LA>
+cudaError_t load_bulk() {
   // idempotent and cheap; avoids per-device bookkeeping
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return cudaFuncSetAttribute(kv_copy_bulk_kernel<W, STAGES, LA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              kRingBytes);
 }
 
 template <int W, int STAGES, int LA>
 cudaError_t launch_bulk(const KvCopyParams& p, int ctas, int tile_bytes, int tiles_per_chunk, cudaStream_t s) {
-  const int smem = W * STAGES * tile_bytes;
-  auto k = kv_copy_bulk_kernel<W, STAGES, LA>;
-  cudaError_t e = ensure_smem(k, smem);
+  cudaError_t e = load_bulk<W, STAGES, LA>();
   if (e != cudaSuccess) return e;
   const int warps = W + (p.layer_major && p.done_counter != nullptr ? 1 : 0);   // last warp = layer signaller
-  k<<<ctas, 32 * warps, smem, s>>>(p, tile_bytes, tiles_per_chunk);
+  kv_copy_bulk_kernel<W, STAGES, LA><<<ctas, 32 * warps, W * STAGES * tile_bytes, s>>>(p, tile_bytes, tiles_per_chunk);
   return cudaGetLastError();
 }
 
@@ -360,6 +363,16 @@ inline bool all_multiple(const KvCopyParams& p, int64_t m) {
 }
 
 }  // namespace
+
+cudaError_t kv_copy_load_kernels() {
+  cudaError_t e = load_bulk<4, 12, 11>();
+  if (e == cudaSuccess) e = load_bulk<4, 12, 6>();
+  if (e == cudaSuccess) e = load_bulk<4, 6, 5>();
+  if (e == cudaSuccess) e = load_bulk<4, 6, 3>();
+  if (e == cudaSuccess) e = load_bulk<4, 3, 2>();
+  if (e == cudaSuccess) e = load_bulk<2, 3, 2>();
+  return e;
+}
 
 bool kv_copy_tma_eligible(const KvCopyParams& p) { return kv_copy_tables_ok(p) && all_multiple(p, 16); }
 

@@ -121,6 +121,9 @@ struct KvCopyLaunch {
 // any multiple of 4 (and single bytes through its tail path).
 cudaError_t launch_kv_copy(const KvCopyParams& p, const KvCopyLaunch& cfg, cudaStream_t stream);
 
+// Loads the bulk kernels into the current device's context, so that the first op does not wait for it.
+cudaError_t kv_copy_load_kernels();
+
 // Re-statement of the reference's copy kernel shape for baseline timing only:
 // 4 CTAs x 1024 threads, one warp per (layer, pair), lanes move 16 bytes
 // (reference: csrc/transfer.cu:95-158,176-190).

@@ -152,6 +152,12 @@ void TransferGroup::rank_main(int r) {
                         cudaHostAllocPortable | cudaHostAllocMapped),
           "cudaHostAlloc(status)");
     for (int i = 0; i < kInflight * kStatusWords; ++i) rk.status[i] = 0;
+    check(kv_copy_load_kernels(), "kv_copy_load_kernels");
+    // the staging buffers are in place before the first op (allocated by it, they cost it 10 to 16 ms)
+    auto may_stage = [](const KvCopyLaunch& c) { return c.engine == kEngineCe || c.engine == kEngineAuto; };
+    if (gpus_.size() == 1 && opt_.ce_staging_blocks != 0 && (may_stage(opt_.h2d) || may_stage(opt_.d2h)) &&
+        host_.block_stride == opt_.chunk_bytes * opt_.kv_dim * opt_.num_layers)
+      ce_staging_prepare(rk.staging, std::max<int64_t>(0, opt_.ce_staging_blocks), host_.block_stride);
   } catch (const std::exception& e) {
     std::lock_guard<std::mutex> g(rk.mu);
     rk.init_error = e.what();
@@ -206,16 +212,21 @@ void TransferGroup::rank_main(int r) {
               if (a.status & (1 << b)) p.status[b] = 1;
             ce_ops_.fetch_add(1, std::memory_order_relaxed);
             done = true;
-          } else if (opt_.ce_staging_blocks > 0 && p.c_block_stride > 0) {
+          } else if (opt_.ce_staging_blocks != 0 && (int)gpus_.size() == 1 &&
+                     ce_host_blocks_abut(p, opt_.num_layers, p.chunk_bytes)) {
             // scattered GPU pages, host blocks in a row: gather into device staging, one large copy per piece
             const int64_t min_run = std::max<int64_t>(1, (opt_.ce_policy.min_bytes_per_copy + p.c_block_stride - 1) /
                                                              p.c_block_stride);
-            std::vector<CeHostRun> runs;
-            if ((int)gpus_.size() == 1 &&
-                ce_host_runs(p, p.gpu_blocks, p.cpu_blocks, p.num_pairs, opt_.num_layers, min_run, runs)) {
+            int64_t* ids = id_ring_ + (size_t)t.slot * 2 * (size_t)opt_.max_blocks_per_op;   // this rank's alone
+            CeStagePlan plan;
+            if (ce_staging_prepare(rk.staging, std::max<int64_t>(0, opt_.ce_staging_blocks), p.c_block_stride) &&
+                ce_plan_staged(p, ids, ids + opt_.max_blocks_per_op, min_run, rk.staging.blocks, plan)) {
               KvCopyLaunch kcfg = cfg;
               kcfg.engine = 0;
-              lerr[i] = ce_copy_staged(p, runs, rk.staging, opt_.ce_staging_blocks, kcfg, rk.stream);
+              lerr[i] = ce_copy_staged(
+                  p, plan, rk.staging,
+                  [&kcfg](const KvCopyParams& q, int64_t, cudaStream_t s) { return launch_kv_copy(q, kcfg, s); },
+                  rk.stream);
               ce_ops_.fetch_add(1, std::memory_order_relaxed);
               staged_ops_.fetch_add(1, std::memory_order_relaxed);
               done = true;

@@ -57,8 +57,8 @@ struct GroupOptions {
   int64_t max_blocks_per_op = 1 << 16;
   bool high_priority_stream = false;
   CePolicy ce_policy;
-  int64_t ce_staging_blocks = 32;   // blocks per staging buffer of the gather + large-copy route (0 = route off);
-                                    // two buffers of this size are allocated per GPU the first time the route runs
+  int64_t ce_staging_blocks = -1;   // blocks per staging buffer of the gather + large-copy route (-1 = kCeStageBytes'
+                                    // worth, 0 = route off)
 };
 
 // Engine selectors of an op (KvCopyLaunch::engine or a per-op override).
@@ -119,7 +119,7 @@ class TransferGroup {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int32_t* status = nullptr;  // mapped pinned word
-    CeStaging staging;          // device staging of the gather + large-copy route (allocated on first use)
+    CeStaging staging;          // device staging of the gather + large-copy route
     bool ready = false;
     std::string init_error;
   };

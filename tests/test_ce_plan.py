@@ -1,6 +1,7 @@
 """Run analysis and routing of the copy-engine path (reference behaviour:
 csrc/ce_transfer.cu:37-104 segments contiguous (gpu, cpu) id runs and picks a path)."""
 import numpy as np
+import pytest
 
 from flexkv_b200 import _native
 
@@ -62,3 +63,39 @@ def test_out_of_range_ids_are_dropped_and_flagged():
     runs, path, copies, status = C.ce_plan(d, 1 << 30, 0)
     assert runs.tolist() == [[1, 1, 2]]
     assert status == 1 | 2      # gpu and cpu range bits
+
+
+@pytest.mark.parametrize("h2d", [0, 1])
+@pytest.mark.parametrize("blocks", [[(5, 1)], [(5, 16), (40, 16)], [(0, 700)], [(9, 300), (900, 1), (400, 15), (1000, 40)],
+                                    [(900, 3), (9, 64), (200, 300), (100, 15)]])
+@pytest.mark.parametrize("max_piece", [1, 7, 128])
+def test_staged_plan_moves_every_pair_once(blocks, max_piece, h2d):
+    """Runs of at least 16 host blocks are staged in pieces, the rest is left over; pairs keep their partners."""
+    c = np.concatenate([np.arange(a, a + n) for a, n in blocks])
+    g = np.random.default_rng(3).permutation(4096)[:c.size]
+    d, keep = _params(g, c, layers=16)                                       # 1 MiB blocks
+    d["h2d"] = h2d
+    plan = C.ce_stage_plan(d, 16, max_piece)
+    longer = [n for _, n in blocks if n >= 16]
+    if not longer or (len(longer) < len(blocks) and sum(longer) < 32):       # mixed ops need 32 MiB in runs
+        assert plan is None
+        return
+    pieces, staged, g2, c2 = plan
+    assert staged == sum(longer)
+    assert sorted(zip(g2.tolist(), c2.tolist())) == sorted(zip(g.tolist(), c.tolist()))
+    seen = []
+    for first, host, m in pieces.tolist():
+        assert 1 <= m <= max_piece
+        assert c2[first:first + m].tolist() == list(range(host, host + m))
+        seen += range(first, first + m)
+    assert sorted(seen) == list(range(staged))
+    small = pieces[-1 if h2d else 0]
+    assert small[2] <= 4                                                     # 4 MiB where the kernel runs alone
+
+
+def test_staged_plan_refuses_ids_out_of_range():
+    for bad in (-1, 4096):
+        g, c = np.arange(64), np.arange(64)
+        c[40] = bad
+        assert C.ce_stage_plan(_params(g, c)[0], 16, 8) is None
+        assert C.ce_stage_plan(_params(c, g)[0], 16, 8) is None

@@ -134,3 +134,38 @@ def test_scattered_pages_with_host_blocks_in_a_row_go_through_the_staging_area()
     gb = g.copy()
     gb[3] = NG + 5
     assert grp.transfer(gb, c, False, 0, shape.num_layers, ENG["auto"]).status == 1
+
+
+@pytest.mark.parametrize("chunk_tokens", [1, 16])
+def test_runs_ride_the_copy_engine_while_stray_host_blocks_stay_with_the_kernel(chunk_tokens):
+    """One op of two long host runs with single blocks between them, in both directions, against the kernel alone."""
+    dev = torch.device("cuda:0")
+    shape = KVShape("t", 5, 8, 128, tokens_per_block=chunk_tokens)     # 2 and 32 KiB chunks, 20 and 320 KiB blocks
+    n_run = {1: 900, 16: 60}[chunk_tokens]
+    NG = NC = 2 * n_run + 40
+    tensors, layout = alloc_paged_cache(shape, NG, dev, "vllm", fill="normal", seed=5)
+    reg = register_tensors(tensors, layout)
+    chunk = reg.chunk_bytes
+    pool = torch.zeros(NC, shape.num_layers, shape.kv_dim, chunk, dtype=torch.uint8).pin_memory()
+    host = dict(base=pool.data_ptr(), layer_stride=shape.kv_dim * chunk, kv_stride=chunk,
+                block_stride=shape.num_layers * shape.kv_dim * chunk, num_blocks=NC)
+    opts = dict(num_layers=shape.num_layers, kv_dim=shape.kv_dim, chunk_bytes=chunk, max_blocks_per_op=4096)
+    grp = C.TransferGroup([reg.as_native()], host, opts)
+    rng = np.random.default_rng(8)
+    c = np.concatenate([[3], np.arange(7, 7 + n_run), [5, 1], np.arange(12 + n_run, 12 + 2 * n_run), [NC - 1]]).astype(np.int64)
+    g = rng.permutation(NG)[:c.size].astype(np.int64)
+    assert grp.transfer(g, c, False, 0, shape.num_layers, ENG["auto"]).status == 0
+    assert grp.staged_ops == 1
+    want = pool.clone()
+    pool.zero_()
+    assert grp.transfer(g, c, False, 0, shape.num_layers, ENG["tma"]).status == 0
+    assert torch.equal(pool, want) and int(want.count_nonzero()) > 0
+    saved = [t.clone() for t in tensors]
+    g2 = rng.permutation(NG)[:c.size].astype(np.int64)
+    for t in tensors:
+        t.zero_()
+    assert grp.transfer(g2, c, True, 0, shape.num_layers, ENG["auto"]).status == 0
+    assert grp.staged_ops == 2
+    a, b = torch.from_numpy(g).to(dev), torch.from_numpy(g2).to(dev)
+    for l in range(shape.num_layers):
+        assert torch.equal(tensors[l][:, b], saved[l][:, a])
