@@ -12,6 +12,7 @@
 #include "kernels/kv_compress.h"
 #include "kernels/kv_hash.h"
 #include "ce_copy.h"
+#include "codec_link.h"
 #include "ptr_table.h"
 #include "ipc.h"
 #include "vmm_handle.h"
@@ -118,6 +119,19 @@ void init_kernel_bindings(py::module_& m) {
     KvCopyParams p = kv_params_from_dict(params);
     throw_on(launch_kv_quant_fp8(p, num_ctas, (cudaStream_t)(uintptr_t)stream), "kv_quant_fp8 launch");
   }, py::arg("params"), py::arg("num_ctas") = 32, py::arg("stream") = (uint64_t)0);
+  py::class_<CodecLink>(m, "CodecLink")
+      .def(py::init<int, int, int, int64_t>(), py::arg("device"), py::arg("num_layers"), py::arg("kv_dim"),
+           py::arg("chunk_slot"), py::call_guard<py::gil_scoped_release>())
+      .def("quant_fp8", [](CodecLink& l, py::dict params, int num_ctas, uint64_t stream) {
+        KvCopyParams p = kv_params_from_dict(params);
+        cudaError_t e;
+        {
+          py::gil_scoped_release rel;
+          e = l.quant_fp8(p, num_ctas, (cudaStream_t)(uintptr_t)stream);
+        }
+        throw_on(e, "kv_quant_fp8");
+      }, py::arg("params"), py::arg("num_ctas"), py::arg("stream"))
+      .def_property_readonly("staged_ops", &CodecLink::staged_ops);
   m.def("fp8_packed_chunk_bytes", &fp8_packed_chunk_bytes);
 
   m.def("kv_compress_bf16", [](py::dict params, uint64_t size_table_ptr, int layers_total, int num_ctas,

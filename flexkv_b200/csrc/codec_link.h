@@ -1,0 +1,41 @@
+// GPU<->host moves of a packed host pool, on the copy engines where the host blocks allow it.
+//
+// The codec kernels read or write the host pool themselves, so their traffic crosses the link as SM-issued requests:
+// 52.5 GB/s out, 51 in, and 37 each way with both directions busy (B200). Where the op's host blocks come in rows the
+// kernel packs into a device staging buffer instead (or unpacks out of it) and a copy engine moves the packed blocks
+// at 56.5 / 55, or 48 each way: the staged route of ce_copy.h with a codec kernel in the place of the plain gather.
+// The packed bytes are the same either way. Blocks that stand alone, pools shared by several ranks of a launch and
+// hosts without memory for the staging buffers stay with the kernel.
+#pragma once
+#include <cstdint>
+
+#include <cuda_runtime.h>
+
+#include "ce_copy.h"
+
+namespace fkv {
+
+// One GPU, one direction. run() is called by one thread at a time.
+class CodecLink {
+ public:
+  // `chunk_slot`: bytes a packed (layer, kv, block) chunk takes in the host pool.
+  CodecLink(int device, int num_layers, int kv_dim, int64_t chunk_slot);
+  ~CodecLink();
+  CodecLink(const CodecLink&) = delete;
+  CodecLink& operator=(const CodecLink&) = delete;
+
+  // Block-scaled fp8, as launch_kv_quant_fp8. `p.gpu_blocks` and `p.cpu_blocks` are host memory that the kernel can
+  // read; their pairs may be reordered. They and the status words are in use until `stream` has passed the op.
+  cudaError_t quant_fp8(const KvCopyParams& p, int num_ctas, cudaStream_t stream);
+  uint64_t staged_ops() const { return staged_ops_; }
+
+ private:
+  bool plan(const KvCopyParams& p, CeStagePlan& out);
+
+  int device_, num_layers_;
+  int64_t chunk_slot_;
+  CeStaging staging_;
+  uint64_t staged_ops_ = 0;
+};
+
+}  // namespace fkv

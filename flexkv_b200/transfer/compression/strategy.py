@@ -4,14 +4,24 @@ A strategy is attached once to a worker (``attach``) and then launches one fused
 pack-or-unpack kernel per rank and op (``run``). Reference plug-in point:
 flexkv/transfer/compression/common/strategy.py:13-51 (``CompressionStrategy.attach/run``,
 ``NullCompressionStrategy``); the nvCOMP ANS strategy of the reference
-(compression/ans/ans_strategy.py) is replaced by own kernels: no staging buffer and no
-second pass, the copy kernel itself reads GPU pages and writes packed host tiles.
+(compression/ans/ans_strategy.py) is replaced by own kernels that read GPU pages and write
+packed tiles, either into the host pool itself or into the staging buffer of a copy-engine move.
 """
 from __future__ import annotations
 
 from typing import Any, Dict
 
 from ... import _native
+
+
+def codec_link(worker: Any):
+    """The native router of a worker's ops between kernel and copy engines, or None where every op belongs to the
+    kernel: an engine of the user's choice (FLEXKV_TRANSFER_ENGINE), or several ranks behind one op, whose slices of a
+    host block are not one span and whose launches read the same id arrays."""
+    if len(worker.regs) != 1 or not worker.copy_engines:
+        return None
+    reg = worker.regs[0]
+    return _native.C.CodecLink(reg.device_id, reg.num_layers, reg.kv_dim, worker.kv_stride)
 
 
 class CompressionStrategy:
@@ -22,6 +32,9 @@ class CompressionStrategy:
 
     def attach(self, worker: Any) -> None:
         self.worker = worker
+
+    def detach(self) -> None:
+        """Gives back what ``attach`` took; no run is in flight."""
 
     def host_chunk_bytes(self, chunk_elems: int, itemsize: int) -> int:
         raise NotImplementedError
@@ -56,8 +69,21 @@ class Fp8BlockScaleStrategy(CompressionStrategy):
             raise ValueError("fp8 offload needs chunk elements divisible by 128")
         return chunk_elems + (chunk_elems // self.GROUP) * 4
 
+    def __init__(self) -> None:
+        self._link = None
+
+    def attach(self, worker) -> None:
+        super().attach(worker)
+        self._link = codec_link(worker)
+
+    def detach(self) -> None:
+        self._link = None
+
     def run(self, params, rank_index, num_ctas, stream) -> None:
-        _native.C.kv_quant_fp8(params, num_ctas, stream)
+        if self._link is not None:
+            self._link.quant_fp8(params, num_ctas, stream)
+        else:
+            _native.C.kv_quant_fp8(params, num_ctas, stream)
 
 
 class ExponentPackStrategy(CompressionStrategy):

@@ -350,12 +350,13 @@ class QuantGpuHostWorker(TransferWorker):
         self.layers_total = self.regs[0].num_layers
         self.shared = model_config.use_mla or model_config.num_kv_heads == 1
         from .compression import build_compressors
-        self.strategy = build_compressors(host, self.layers_total, self.regs[0].kv_dim, len(self.regs), self.shared)
-        self.strategy.attach(self)
         n = 1 if self.shared else model_config.effective_tp_size
         self.host = host
         self.layer_stride, self.kv_stride, self.tp_stride = host.layer_stride // n, host.kv_stride // n, \
             host.block_bytes // n
+        self.copy_engines = _launch_cfg(GLOBAL_CONFIG_FROM_ENV, h2d)["engine"] >= _ENGINE_IDS["ce"]
+        self.strategy = build_compressors(host, self.layers_total, self.regs[0].kv_dim, len(self.regs), self.shared)
+        self.strategy.attach(self)
         # Tile pipelines per launch (two share an SM in the lossless codec's kernel). Measured on B200 with
         # Llama-3-8B blocks: 80 pipelines (40 SMs) put both directions on the link's plateau for SM-issued
         # traffic; the fp8 kernel needs fewer (its CTAs are single pipelines)
@@ -364,6 +365,9 @@ class QuantGpuHostWorker(TransferWorker):
         self._torch = torch
         self.streams = {r.device_id: torch.cuda.Stream(device=r.device_id) for r in self.regs}
         self.status = {r.device_id: torch.zeros(8, dtype=torch.int32, device=f"cuda:{r.device_id}") for r in self.regs}
+
+    def close(self) -> None:
+        self.strategy.detach()
 
     def execute(self, op: TransferOp) -> OpOutcome:
         torch = self._torch

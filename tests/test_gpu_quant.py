@@ -5,9 +5,9 @@ import numpy as np
 import pytest
 import torch
 
-from flexkv_b200 import CacheConfig, KVManager
+from flexkv_b200 import CacheConfig, KVManager, _native
 from flexkv_b200.models import KVShape, alloc_paged_cache, make_model_config
-from flexkv_b200.ops.kv_copy import HostSide, decode_status, new_status
+from flexkv_b200.ops.kv_copy import HostSide, decode_status, make_params, new_status
 from flexkv_b200.ops.kv_quant import kv_quant_fp8, packed_chunk_bytes, reference_pack, reference_unpack
 from flexkv_b200.storage.gpu_layout import register_tensors
 
@@ -64,6 +64,50 @@ def test_pack_unpack_match_reference(shape):
             err = (got.float() - orig.float()).abs().reshape(n, -1, 128).amax(-1)
             bound = orig.float().abs().reshape(n, -1, 128).amax(-1) / 16 + 1e-30
             assert bool((err <= bound).all())
+
+
+@pytest.mark.parametrize("shape", [KVShape("l1", 16, 8, 128, tokens_per_block=16),
+                                   KVShape("l2", 15, 1, 576, use_mla=True, tokens_per_block=64)])   # ragged last tile
+def test_copy_engine_route_moves_the_same_bytes(shape):
+    """Host runs through the staging buffer, stray host blocks by the kernel, in one op; against the kernel alone."""
+    dev = torch.device("cuda:0")
+    n_run = 70
+    NB = 2 * n_run + 20
+    kv, layout = alloc_paged_cache(shape, NB, dev, "vllm", fill="normal", seed=63)
+    reg = register_tensors(kv, layout)
+    pc = packed_chunk_bytes(reg.chunk_bytes // 2)
+    L, K = shape.num_layers, shape.kv_dim
+    pool = torch.zeros(NB, L * K * pc, dtype=torch.uint8).pin_memory()
+    rng = np.random.default_rng(5)
+    c = np.concatenate([[2], np.arange(5, 5 + n_run), [4, 0], np.arange(8 + n_run, 8 + 2 * n_run)]).astype(np.int64)
+    g = rng.permutation(NB)[:c.size].astype(np.int64)
+    g2 = rng.permutation(NB)[:c.size].astype(np.int64)
+    host = HostSide(pool.data_ptr(), K * pc, pc, L * K * pc, NB)
+    status = new_status(dev)
+    keep = kv_quant_fp8(reg, host, g, c, h2d=False, status=status)
+    torch.cuda.synchronize()
+    want = pool.clone()
+    assert int(want.count_nonzero()) > 0
+    for h2d, pages in ((False, g), (True, g2)):
+        link = _native.C.CodecLink(0, L, K, pc)
+        ids = [torch.from_numpy(a.copy()).pin_memory() for a in (pages, c)]
+        if h2d:
+            saved = [t.clone() for t in kv]
+            keep += kv_quant_fp8(reg, host, pages, c, h2d=True, status=status)
+            torch.cuda.synchronize()
+            restored = [t.clone() for t in kv]
+            for t, s in zip(kv, saved):
+                t.copy_(s)
+        else:
+            pool.zero_()
+        link.quant_fp8(make_params(reg, host, *ids, h2d, status_ptr=status.data_ptr()), 32,
+                       torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert link.staged_ops == 1 and decode_status(status) == 0
+        if h2d:
+            assert all(torch.equal(t.view(torch.int16), r.view(torch.int16)) for t, r in zip(kv, restored))
+        else:
+            assert torch.equal(pool, want)
 
 
 def test_kvmanager_with_fp8_host_pool_halves_the_host_block():
