@@ -119,9 +119,14 @@ void init_kernel_bindings(py::module_& m) {
     KvCopyParams p = kv_params_from_dict(params);
     throw_on(launch_kv_quant_fp8(p, num_ctas, (cudaStream_t)(uintptr_t)stream), "kv_quant_fp8 launch");
   }, py::arg("params"), py::arg("num_ctas") = 32, py::arg("stream") = (uint64_t)0);
+  // the codec kernels, loaded into the current device's context
+  m.def("codec_load_kernels", [] {
+    throw_on(kv_quant_load_kernels(), "kv_quant_load_kernels");
+    throw_on(kv_compress_load_kernels(), "kv_compress_load_kernels");
+  });
   py::class_<CodecLink>(m, "CodecLink")
-      .def(py::init<int, int, int, int64_t>(), py::arg("device"), py::arg("num_layers"), py::arg("kv_dim"),
-           py::arg("chunk_slot"), py::call_guard<py::gil_scoped_release>())
+      .def(py::init<int, int, int, int64_t, int64_t>(), py::arg("device"), py::arg("num_layers"), py::arg("kv_dim"),
+           py::arg("chunk_slot"), py::arg("staging_bytes") = kCeStageBytes, py::call_guard<py::gil_scoped_release>())
       .def("quant_fp8", [](CodecLink& l, py::dict params, int num_ctas, uint64_t stream) {
         KvCopyParams p = kv_params_from_dict(params);
         cudaError_t e;
@@ -131,6 +136,17 @@ void init_kernel_bindings(py::module_& m) {
         }
         throw_on(e, "kv_quant_fp8");
       }, py::arg("params"), py::arg("num_ctas"), py::arg("stream"))
+      .def("compress_bf16", [](CodecLink& l, py::dict params, uint64_t size_table_ptr, int layers_total, int num_ctas,
+                               uint64_t stream) {
+        KvCopyParams p = kv_params_from_dict(params);
+        cudaError_t e;
+        {
+          py::gil_scoped_release rel;
+          e = l.compress_bf16(p, (uint32_t*)(uintptr_t)size_table_ptr, layers_total, num_ctas,
+                              (cudaStream_t)(uintptr_t)stream);
+        }
+        throw_on(e, "kv_compress_bf16");
+      }, py::arg("params"), py::arg("size_table_ptr"), py::arg("layers_total"), py::arg("num_ctas"), py::arg("stream"))
       .def_property_readonly("staged_ops", &CodecLink::staged_ops);
   m.def("fp8_packed_chunk_bytes", &fp8_packed_chunk_bytes);
 

@@ -159,7 +159,7 @@ bool ce_host_blocks_abut(const KvCopyParams& p, int total_layers, int64_t chunk_
 }
 
 bool ce_plan_staged(const KvCopyParams& p, int64_t* g, int64_t* c, int64_t min_run, int64_t max_piece,
-                    CeStagePlan& plan) {
+                    CeStagePlan& plan, int64_t ramp_bytes) {
   plan.pieces.clear();
   plan.staged = 0;
   const int64_t n = p.num_pairs;
@@ -194,7 +194,7 @@ bool ce_plan_staged(const KvCopyParams& p, int64_t* g, int64_t* c, int64_t min_r
   // Small pieces where the kernel runs alone: first in an offload, last in a restore. Otherwise a run is cut evenly: a
   // large piece is gathered while the one before it crosses the link, and behind a short remainder the link would
   // wait (host runs of 14 to 49 blocks, pieces of at most 15, B200: 53.2 GB/s with remainders of 1 to 4, 56.5 evenly).
-  int64_t next = std::min(max_piece, std::max<int64_t>(1, kCeRampBytes / p.c_block_stride));
+  int64_t next = std::min(max_piece, std::max<int64_t>(1, ramp_bytes / p.c_block_stride));
   auto cut = [&](const CeHostRun& r) {
     for (int64_t done = 0; done < r.len;) {
       const int64_t rest = r.len - done;
@@ -222,23 +222,32 @@ bool ce_plan_staged(const KvCopyParams& p, int64_t* g, int64_t* c, int64_t min_r
 }
 
 cudaError_t ce_copy_staged(const KvCopyParams& p, const CeStagePlan& plan, CeStaging& st, const CeStageKernel& kernel,
-                           cudaStream_t stream) {
+                           cudaStream_t stream, const CeLinkCopy* link) {
   const int64_t block_bytes = p.c_block_stride;
   cudaError_t e = cudaSuccess;
-  auto others = [&]() -> cudaError_t {
-    if (plan.staged >= p.num_pairs) return cudaSuccess;
+  auto by_kernel = [&](int64_t first, int64_t pairs) -> cudaError_t {
+    if (pairs <= 0) return cudaSuccess;
     KvCopyParams q = p;
-    q.gpu_blocks = p.gpu_blocks + plan.staged;
-    q.cpu_blocks = p.cpu_blocks + plan.staged;
-    q.num_pairs = (int32_t)(p.num_pairs - plan.staged);
+    q.gpu_blocks = p.gpu_blocks + first;
+    q.cpu_blocks = p.cpu_blocks + first;
+    q.num_pairs = (int32_t)pairs;
     return kernel(q, 0, stream);
   };
-  if (p.h2d) e = others();
+  auto link_copy = [&](const CeHostRun& piece, uint8_t* staged) -> cudaError_t {
+    if (link) return link->copy(piece, staged, st.copy_stream);
+    void* host = reinterpret_cast<uint8_t*>(p.cpu_base) + piece.cpu_block * block_bytes;
+    const size_t bytes = (size_t)(piece.len * block_bytes);
+    return p.h2d ? cudaMemcpyAsync(staged, host, bytes, cudaMemcpyHostToDevice, st.copy_stream)
+                 : cudaMemcpyAsync(host, staged, bytes, cudaMemcpyDeviceToHost, st.copy_stream);
+  };
+  if (p.h2d) e = by_kernel(plan.staged, p.num_pairs - plan.staged);
   int b = 0;
   for (const CeHostRun& piece : plan.pieces) {
     if (e != cudaSuccess) return e;
-    uint8_t* host = reinterpret_cast<uint8_t*>(p.cpu_base) + piece.cpu_block * block_bytes;
-    const size_t bytes = (size_t)(piece.len * block_bytes);
+    if (link && !link->worth(piece)) {
+      e = by_kernel(piece.first, piece.len);
+      continue;
+    }
     KvCopyParams q = p;            // the staging buffer plays the host side, in host block format
     q.cpu_base = reinterpret_cast<uint64_t>(st.buf[b]);
     q.gpu_blocks = p.gpu_blocks + piece.first;
@@ -254,12 +263,12 @@ cudaError_t ce_copy_staged(const KvCopyParams& p, const CeStagePlan& plan, CeSta
       if (e == cudaSuccess) e = kernel(q, piece.cpu_block, stream);
       if (e == cudaSuccess) e = cudaEventRecord(st.kernel_done[b], stream);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(st.copy_stream, st.kernel_done[b], 0);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(host, st.buf[b], bytes, cudaMemcpyDeviceToHost, st.copy_stream);
+      if (e == cudaSuccess) e = link_copy(piece, st.buf[b]);
       if (e == cudaSuccess) e = cudaEventRecord(st.copy_done[b], st.copy_stream);
     } else {
       // one large copy in once the previous scatter out of this buffer is done, then the scatter kernel
       if (st.used[b]) e = cudaStreamWaitEvent(st.copy_stream, st.kernel_done[b], 0);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(st.buf[b], host, bytes, cudaMemcpyHostToDevice, st.copy_stream);
+      if (e == cudaSuccess) e = link_copy(piece, st.buf[b]);
       if (e == cudaSuccess) e = cudaEventRecord(st.copy_done[b], st.copy_stream);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, st.copy_done[b], 0);
       if (e == cudaSuccess) e = kernel(q, piece.cpu_block, stream);
@@ -268,7 +277,7 @@ cudaError_t ce_copy_staged(const KvCopyParams& p, const CeStagePlan& plan, CeSta
     if (e == cudaSuccess) st.used[b] = true;
     b = b + 1 == kCeStageBufs ? 0 : b + 1;
   }
-  if (!p.h2d && e == cudaSuccess) e = others();
+  if (!p.h2d && e == cudaSuccess) e = by_kernel(plan.staged, p.num_pairs - plan.staged);
   // the caller's stream ends after the last copies
   for (b = 0; b < kCeStageBufs && e == cudaSuccess; ++b)
     if (st.used[b]) e = cudaStreamWaitEvent(stream, st.copy_done[b], 0);

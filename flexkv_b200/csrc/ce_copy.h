@@ -110,16 +110,22 @@ bool ce_host_blocks_abut(const KvCopyParams& p, int total_layers, int64_t chunk_
 // first) and the op is only split when the runs hold at least kCeMixedMinBytes. False, with the arrays as they were,
 // when the op belongs to the kernel: an id out of range, no run long enough.
 bool ce_plan_staged(const KvCopyParams& p, int64_t* gpu_blocks, int64_t* cpu_blocks, int64_t min_run,
-                    int64_t max_piece, CeStagePlan& plan);
+                    int64_t max_piece, CeStagePlan& plan, int64_t ramp_bytes = kCeRampBytes);
 
 // Launches the kernel of a piece or of the pairs that stay with it. For a piece, `q` addresses the staging buffer as
 // the host side (block ids 0, 1, ...) and `host_block` is the host block that id 0 stands for; otherwise it is 0.
 using CeStageKernel = std::function<cudaError_t(const KvCopyParams& q, int64_t host_block, cudaStream_t stream)>;
+// Moves a staged piece to or from the host where that is not one contiguous copy of its blocks. `worth` is asked
+// before anything is queued for the piece; a piece that it declines is left to the kernel.
+struct CeLinkCopy {
+  std::function<bool(const CeHostRun& piece)> worth;
+  std::function<cudaError_t(const CeHostRun& piece, uint8_t* staged, cudaStream_t stream)> copy;
+};
 // Moves the op: pieces through the staging buffers, gather or scatter kernel on `stream`, large copies on the
 // staging's own stream, both buffers in flight; the other pairs by the kernel, on `stream`, beside the last copies
 // (offload) or the first ones (restore). When it returns, everything has been queued and `stream` waits for the last
 // copy. `p` carries the id arrays as planned.
 cudaError_t ce_copy_staged(const KvCopyParams& p, const CeStagePlan& plan, CeStaging& st, const CeStageKernel& kernel,
-                           cudaStream_t stream);
+                           cudaStream_t stream, const CeLinkCopy* link = nullptr);
 
 }  // namespace fkv

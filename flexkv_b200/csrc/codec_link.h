@@ -18,8 +18,9 @@ namespace fkv {
 // One GPU, one direction. run() is called by one thread at a time.
 class CodecLink {
  public:
-  // `chunk_slot`: bytes a packed (layer, kv, block) chunk takes in the host pool.
-  CodecLink(int device, int num_layers, int kv_dim, int64_t chunk_slot);
+  // `chunk_slot`: bytes a packed (layer, kv, block) chunk takes in the host pool; `staging_bytes` of each of the two
+  // staging buffers.
+  CodecLink(int device, int num_layers, int kv_dim, int64_t chunk_slot, int64_t staging_bytes = kCeStageBytes);
   ~CodecLink();
   CodecLink(const CodecLink&) = delete;
   CodecLink& operator=(const CodecLink&) = delete;
@@ -27,13 +28,19 @@ class CodecLink {
   // Block-scaled fp8, as launch_kv_quant_fp8. `p.gpu_blocks` and `p.cpu_blocks` are host memory that the kernel can
   // read; their pairs may be reordered. They and the status words are in use until `stream` has passed the op.
   cudaError_t quant_fp8(const KvCopyParams& p, int num_ctas, cudaStream_t stream);
+  // The lossless codec, as launch_kv_compress_bf16; `size_table` is host memory that the kernel can read. Restores are
+  // staged: only the used bytes of the tile slots cross, as rows of a 2-D copy, each class of tiles (K or V, tile of
+  // the chunk) as wide as its largest tile in the piece. Offloads stay with the kernel: the sizes are not known before
+  // a piece is packed, and rows of 11 KiB go out at 51.7 GB/s where the kernel reaches 52.5.
+  cudaError_t compress_bf16(const KvCopyParams& p, uint32_t* size_table, int layers_total, int num_ctas,
+                            cudaStream_t stream);
   uint64_t staged_ops() const { return staged_ops_; }
 
  private:
-  bool plan(const KvCopyParams& p, CeStagePlan& out);
+  bool plan(const KvCopyParams& p, int64_t min_bytes, int64_t ramp_bytes, CeStagePlan& out);
 
   int device_, num_layers_;
-  int64_t chunk_slot_;
+  int64_t chunk_slot_, staging_bytes_;
   CeStaging staging_;
   uint64_t staged_ops_ = 0;
 };

@@ -571,7 +571,19 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
   }
 }
 
+// host reads need several tiles in flight per pipeline to cover the PCIe round trip
+constexpr int kInUnpack = 4, kInPack = 3;
+constexpr int kSmemUnpack = (int)sizeof(Smem<kInUnpack>) * kGroups + 128;
+constexpr int kSmemPack = (int)sizeof(Smem<kInPack>) * kGroups + 128;
+
 }  // namespace
+
+cudaError_t kv_compress_load_kernels() {
+  const cudaError_t e = cudaFuncSetAttribute(kv_compress_kernel<false, kInUnpack>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemUnpack);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(kv_compress_kernel<true, kInPack>,
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPack);
+}
 
 cudaError_t launch_kv_compress_bf16(const KvCopyParams& p, uint32_t* size_table, int layers_total, int num_ctas,
                                     cudaStream_t stream) {
@@ -586,23 +598,14 @@ cudaError_t launch_kv_compress_bf16(const KvCopyParams& p, uint32_t* size_table,
   int64_t pipes = num_ctas > 0 ? num_ctas : 32;
   if (pipes > total) pipes = total;
   const int ctas = (int)((pipes + kGroups - 1) / kGroups);
-  cudaError_t e;
-  if (p.h2d) {
-    // host reads need several tiles in flight per pipeline to cover the PCIe round trip
-    constexpr int kIn = 4;
-    const int smem = (int)sizeof(Smem<kIn>) * kGroups + 128;
-    e = cudaFuncSetAttribute(kv_compress_kernel<false, kIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    kv_compress_kernel<false, kIn><<<ctas, kThreads * kGroups, smem, stream>>>(p, size_table, layers_total,
-                                                                               tiles_per_chunk);
-  } else {
-    constexpr int kIn = 3;
-    const int smem = (int)sizeof(Smem<kIn>) * kGroups + 128;
-    e = cudaFuncSetAttribute(kv_compress_kernel<true, kIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    kv_compress_kernel<true, kIn><<<ctas, kThreads * kGroups, smem, stream>>>(p, size_table, layers_total,
-                                                                              tiles_per_chunk);
-  }
+  const cudaError_t e = kv_compress_load_kernels();
+  if (e != cudaSuccess) return e;
+  if (p.h2d)
+    kv_compress_kernel<false, kInUnpack><<<ctas, kThreads * kGroups, kSmemUnpack, stream>>>(p, size_table, layers_total,
+                                                                                            tiles_per_chunk);
+  else
+    kv_compress_kernel<true, kInPack><<<ctas, kThreads * kGroups, kSmemPack, stream>>>(p, size_table, layers_total,
+                                                                                       tiles_per_chunk);
   return cudaGetLastError();
 }
 

@@ -71,4 +71,7 @@ inline int64_t compress_chunk_slot_bytes(int64_t chunk_elems) {
 cudaError_t launch_kv_compress_bf16(const KvCopyParams& p, uint32_t* size_table, int layers_total, int num_ctas,
                                     cudaStream_t stream);
 
+// Loads the kernels into the current device's context, so that the first op does not wait for it.
+cudaError_t kv_compress_load_kernels();
+
 }  // namespace fkv

@@ -222,6 +222,13 @@ __global__ void __launch_bounds__(kThreads, 2) kv_quant_fp8_kernel(const __grid_
 
 }  // namespace
 
+cudaError_t kv_quant_load_kernels() {
+  const cudaError_t e = cudaFuncSetAttribute(kv_quant_fp8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(Smem<false>));
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(kv_quant_fp8_kernel<true>,
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<true>));
+}
+
 cudaError_t launch_kv_quant_fp8(const KvCopyParams& p, int num_ctas, cudaStream_t stream) {
   if (p.num_pairs <= 0 || p.num_layers <= 0 || p.kv_dim <= 0 || p.chunk_bytes <= 0) return cudaSuccess;
   const int64_t chunk_elems = p.chunk_bytes / 2;
@@ -230,18 +237,12 @@ cudaError_t launch_kv_quant_fp8(const KvCopyParams& p, int num_ctas, cudaStream_
   const int64_t total = (int64_t)p.num_pairs * p.num_layers * p.kv_dim * tiles_per_chunk;
   int ctas = num_ctas > 0 ? num_ctas : 32;
   if ((int64_t)ctas > total) ctas = (int)total;
-  cudaError_t e;
-  if (p.h2d) {
-    constexpr int smem = (int)sizeof(Smem<false>);
-    e = cudaFuncSetAttribute(kv_quant_fp8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    kv_quant_fp8_kernel<false><<<ctas, kThreads, smem, stream>>>(p, tiles_per_chunk);
-  } else {
-    constexpr int smem = (int)sizeof(Smem<true>);
-    e = cudaFuncSetAttribute(kv_quant_fp8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    kv_quant_fp8_kernel<true><<<ctas, kThreads, smem, stream>>>(p, tiles_per_chunk);
-  }
+  const cudaError_t e = kv_quant_load_kernels();
+  if (e != cudaSuccess) return e;
+  if (p.h2d)
+    kv_quant_fp8_kernel<false><<<ctas, kThreads, sizeof(Smem<false>), stream>>>(p, tiles_per_chunk);
+  else
+    kv_quant_fp8_kernel<true><<<ctas, kThreads, sizeof(Smem<true>), stream>>>(p, tiles_per_chunk);
   return cudaGetLastError();
 }
 

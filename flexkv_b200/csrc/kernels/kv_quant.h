@@ -27,4 +27,7 @@ inline int64_t fp8_packed_chunk_bytes(int64_t chunk_elems) { return chunk_elems 
 // those of the packed format. p.h2d selects unpack (1) or pack (0).
 cudaError_t launch_kv_quant_fp8(const KvCopyParams& p, int num_ctas, cudaStream_t stream);
 
+// Loads the kernels into the current device's context, so that the first op does not wait for it.
+cudaError_t kv_quant_load_kernels();
+
 }  // namespace fkv

@@ -14,14 +14,14 @@ from typing import Any, Dict
 from ... import _native
 
 
-def codec_link(worker: Any):
+def codec_link(worker: Any, staging_bytes: int):
     """The native router of a worker's ops between kernel and copy engines, or None where every op belongs to the
     kernel: an engine of the user's choice (FLEXKV_TRANSFER_ENGINE), or several ranks behind one op, whose slices of a
     host block are not one span and whose launches read the same id arrays."""
     if len(worker.regs) != 1 or not worker.copy_engines:
         return None
     reg = worker.regs[0]
-    return _native.C.CodecLink(reg.device_id, reg.num_layers, reg.kv_dim, worker.kv_stride)
+    return _native.C.CodecLink(reg.device_id, reg.num_layers, reg.kv_dim, worker.kv_stride, staging_bytes)
 
 
 class CompressionStrategy:
@@ -74,7 +74,7 @@ class Fp8BlockScaleStrategy(CompressionStrategy):
 
     def attach(self, worker) -> None:
         super().attach(worker)
-        self._link = codec_link(worker)
+        self._link = codec_link(worker, 32 << 20)
 
     def detach(self) -> None:
         self._link = None
@@ -97,6 +97,15 @@ class ExponentPackStrategy(CompressionStrategy):
     def __init__(self, size_table=None, spec=None) -> None:
         self.size_table = size_table
         self.spec = spec
+        self._link = None
+
+    def attach(self, worker) -> None:
+        super().attach(worker)
+        # restores only; rows of about 1000 tiles per copy need a larger buffer than whole blocks do
+        self._link = codec_link(worker, 64 << 20) if worker.h2d else None
+
+    def detach(self) -> None:
+        self._link = None
 
     @property
     def needs_size_table(self) -> bool:
@@ -112,8 +121,11 @@ class ExponentPackStrategy(CompressionStrategy):
         if self.size_table is None or self.spec is None:
             raise RuntimeError("exponent-packing strategy used without a size table")
         off = self.spec.rank_offset_entries(rank_index)
-        _native.C.kv_compress_bf16(params, self.size_table.data_ptr() + 4 * off, self.spec.kernel_layers(), num_ctas,
-                                   stream)
+        table, layers = self.size_table.data_ptr() + 4 * off, self.spec.kernel_layers()
+        if self._link is not None:
+            self._link.compress_bf16(params, table, layers, num_ctas, stream)
+        else:
+            _native.C.kv_compress_bf16(params, table, layers, num_ctas, stream)
 
 
 def strategy_for(codec: str, size_table=None, spec=None) -> CompressionStrategy:

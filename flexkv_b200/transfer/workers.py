@@ -365,6 +365,9 @@ class QuantGpuHostWorker(TransferWorker):
         self._torch = torch
         self.streams = {r.device_id: torch.cuda.Stream(device=r.device_id) for r in self.regs}
         self.status = {r.device_id: torch.zeros(8, dtype=torch.int32, device=f"cuda:{r.device_id}") for r in self.regs}
+        for r in self.regs:
+            with torch.cuda.device(r.device_id):
+                _native.C.codec_load_kernels()
 
     def close(self) -> None:
         self.strategy.detach()

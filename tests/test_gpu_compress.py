@@ -5,11 +5,12 @@ import numpy as np
 import pytest
 import torch
 
+from flexkv_b200 import _native
 from flexkv_b200.models import KVShape, alloc_paged_cache
 from flexkv_b200.ops.kv_compress import (TILE_ELEMS, TILE_SLOT, chunk_slot_bytes, kv_compress,
                                          reference_compress_tile, reference_decompress_tile, size_table_entries,
                                          tiles_per_chunk)
-from flexkv_b200.ops.kv_copy import HostSide, decode_status, new_status
+from flexkv_b200.ops.kv_copy import HostSide, decode_status, make_params, new_status
 from flexkv_b200.storage.gpu_layout import register_tensors
 
 pytestmark = pytest.mark.gpu
@@ -147,3 +148,57 @@ def test_kvmanager_with_lossless_codec_host_and_ssd(tmp_path):
                 assert torch.equal(kv[l][:, di].view(torch.int16), saved[l][:, si].view(torch.int16))
     finally:
         mgr.shutdown()
+
+
+@pytest.mark.parametrize("shape,spread", [(KVShape("r1", 16, 8, 128, tokens_per_block=16), False),   # two full tiles a chunk
+                                          (KVShape("r1", 16, 8, 128, tokens_per_block=16), True),    # some tiles raw
+                                          (KVShape("r2", 15, 1, 576, use_mla=True, tokens_per_block=64), False),
+                                          (KVShape("r3", 48, 1, 128, tokens_per_block=16), False)])  # 3 KiB rows
+def test_restore_through_the_copy_engines_matches_the_kernel(shape, spread):
+    """Host runs come in as rows of the used bytes, stray blocks by the kernel; a piece whose tiles differ much in
+    size stays with the kernel. Tiles beyond the used bytes are never looked at: the slots hold garbage there."""
+    dev = torch.device("cuda:0")
+    n_run = 70 if shape.num_layers < 48 else 200
+    NB = 2 * n_run + 20
+    kv, layout = alloc_paged_cache(shape, NB, dev, "vllm", fill="normal", seed=71)
+    if not shape.use_mla:
+        for t in kv:
+            t[0].mul_(torch.exp(torch.randn(t.shape[-1], device=dev)))          # keys pack worse than values
+    if spread:
+        kv[3].view(torch.int16).random_(-32768, 32767)
+    reg = register_tensors(kv, layout)
+    E = reg.chunk_bytes // 2
+    slot = chunk_slot_bytes(E)
+    L, K = shape.num_layers, shape.kv_dim
+    pool = torch.full((NB, L * K * slot), 255, dtype=torch.uint8).pin_memory()
+    table = torch.zeros(size_table_entries(NB, L, K, E), dtype=torch.int32).pin_memory()
+    host = HostSide(pool.data_ptr(), K * slot, slot, L * K * slot, NB)
+    rng = np.random.default_rng(6)
+    c = np.concatenate([[2], np.arange(5, 5 + n_run), [4, 0], np.arange(8 + n_run, 8 + 2 * n_run)]).astype(np.int64)
+    g = rng.permutation(NB)[:c.size].astype(np.int64)
+    status = new_status(dev)
+    keep = kv_compress(reg, host, table, g, c, h2d=False, num_ctas=80, status=status)
+    torch.cuda.synchronize()
+    saved = [t.clone() for t in kv]
+    for t in kv:
+        t.zero_()
+    g2 = rng.permutation(NB)[:c.size].astype(np.int64)
+    ids = [torch.from_numpy(a.copy()).pin_memory() for a in (g2, c)]
+    link = _native.C.CodecLink(0, L, K, slot, 8 << 20)
+    link.compress_bf16(make_params(reg, host, *ids, True, status_ptr=status.data_ptr()), table.data_ptr(), L, 80,
+                       torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert decode_status(status) == 0 and link.staged_ops == 1
+    a, b = torch.from_numpy(g).to(dev), torch.from_numpy(g2).to(dev)
+    other = torch.ones(NB, dtype=torch.bool)
+    other[g2] = False
+    for t, s in zip(kv, saved):
+        t, s = (t.unsqueeze(0), s.unsqueeze(0)) if shape.use_mla else (t, s)
+        assert torch.equal(t[:, b].view(torch.int16), s[:, a].view(torch.int16))
+        assert not bool(t[:, other.to(dev)].view(torch.int16).any())
+    # a slot that was never written: every size that is there is restored, the error is reported
+    table.view(NB, -1)[c[10], 3] = 0
+    link.compress_bf16(make_params(reg, host, *ids, True, status_ptr=status.data_ptr()), table.data_ptr(), L, 80,
+                       torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert decode_status(status) == 16
