@@ -83,6 +83,10 @@ void LayerwiseGroup::start_ranks() {
   if (gpus_.empty()) throw std::invalid_argument("LayerwiseGroup: no GPUs");
   if (opt_.num_counters < 1 || opt_.layers_per_batch < -1) throw std::invalid_argument("LayerwiseGroup: bad options");
   const int L = opt_.group.num_layers, R = (int)gpus_.size(), C = opt_.num_counters;
+  if (opt_.group.h2d.engine >= kEngineCe) {      // names of the router, which the kernel launcher does not know
+    opt_.group.h2d.engine = kEngineTma;
+    copy_engines_ = mgroups_.empty() && opt_.size_table == nullptr && opt_.layers_per_batch < 0;
+  }
   epochs_.assign((size_t)C, 0);
   reserved_.assign((size_t)C, 0);
   launched_.assign((size_t)C * gpus_.size(), 0);
@@ -278,6 +282,8 @@ void LayerwiseGroup::rank_main(int r) {
     rk.layer_ev.resize((size_t)C * L);
     for (auto& e : rk.layer_ev) check(cudaEventCreate(&e), "cudaEventCreate");
     check(cudaEventCreate(&rk.ev_begin), "cudaEventCreate");
+    check(kv_copy_load_kernels(), "kv_copy_load_kernels");
+    if (copy_engines_) ce_staging_prepare(rk.staging, 0, opt_.group.chunk_bytes * opt_.group.kv_dim);
     check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
   } catch (const std::exception& e) {
     std::lock_guard<std::mutex> g(rk.mu);
@@ -302,6 +308,7 @@ void LayerwiseGroup::rank_main(int r) {
     done_cv_.notify_all();
   }
   for (auto& e : rk.layer_ev) cudaEventDestroy(e);
+  ce_staging_free(rk.staging);
   if (rk.ev_begin) cudaEventDestroy(rk.ev_begin);
   if (rk.dev_flags) cudaFree(rk.dev_flags);
   if (rk.done_counter) cudaFree(rk.done_counter);
@@ -340,6 +347,78 @@ cudaError_t LayerwiseGroup::stage_ids(Rank& rk, const Job& j, const int64_t*& gp
     cpu_ids = rk.dev_ids + half;
   }
   return err;
+}
+
+// One layer per copy and scatter. B200, GB/s: rows of 64 KiB come in at 54.7 (50.3 where a copy has 32 of them), rows of
+// 8 KiB at 48.7, the layer-major kernel reads 51; a copy costs 3.5 us beside its bytes.
+constexpr int64_t kLayerMinBytes = 6 << 20, kLayerMinRowBytes = 16 << 10, kLayerMinRunBytes = 2 << 20;
+
+bool LayerwiseGroup::plan_staged(Rank& rk, const Job& j, const KvCopyParams& p, std::vector<CeHostRun>& runs) {
+  const int64_t row = p.chunk_bytes * p.kv_dim, layer = row * j.n;
+  if (!copy_engines_ || p.c_use_table || (p.kv_dim > 1 && p.c_kv_stride != p.chunk_bytes) || p.c_block_stride < row ||
+      row < kLayerMinRowBytes || layer < kLayerMinBytes || rk.staging.block_bytes != row || !kv_copy_tables_ok(p))
+    return false;
+  runs.clear();
+  for (int64_t i = 0; i < j.n; ++i) {
+    const int64_t g = j.gpu_blocks[i], c = j.cpu_blocks[i];
+    if (p.gpu_num_blocks > 0 && (g < 0 || g >= p.gpu_num_blocks)) return false;
+    if (p.cpu_num_blocks > 0 && (c < 0 || c >= p.cpu_num_blocks)) return false;
+    if (!runs.empty() && c == runs.back().cpu_block + runs.back().len) ++runs.back().len;
+    else runs.push_back(CeHostRun{i, c, 1});
+  }
+  return layer / (int64_t)runs.size() >= kLayerMinRunBytes;
+}
+
+cudaError_t LayerwiseGroup::queue_staged(int r, const Job& j, const int64_t* gpu_ids, const std::vector<CeHostRun>& runs) {
+  Rank& rk = *ranks_[(size_t)r];
+  CeStaging& st = rk.staging;
+  const int L = opt_.group.num_layers, R = (int)gpus_.size();
+  const int64_t parts = (j.n + st.blocks - 1) / st.blocks, per = (j.n + parts - 1) / parts;
+  cudaEvent_t* ev = rk.layer_ev.data() + (size_t)j.counter * L;
+  // the copies overtake nothing that was queued before this restore
+  cudaError_t e = cudaStreamWaitEvent(st.copy_stream, rk.ev_begin, 0);
+  int b = 0;
+  for (int l = 0; l < L && e == cudaSuccess; ++l) {
+    KvCopyParams p;
+    bool skip = false;
+    fill_kv_params(gpus_[(size_t)r], host_, opt_.group, r, R, gpu_ids, st.iota, j.n, true, l, 1, 0, p, skip);
+    p.status = rk.status;
+    const int64_t row = p.chunk_bytes * p.kv_dim;
+    const uint8_t* host = reinterpret_cast<const uint8_t*>(p.cpu_base) + l * p.c_layer_stride + p.c_off;
+    for (int64_t lo = 0; lo < j.n && e == cudaSuccess; lo += per) {
+      const int64_t hi = std::min(j.n, lo + per);
+      if (st.used[b]) e = cudaStreamWaitEvent(st.copy_stream, st.kernel_done[b], 0);
+      for (const CeHostRun& run : runs) {
+        const int64_t a = std::max(lo, run.first), z = std::min(hi, run.first + run.len);
+        if (a >= z || e != cudaSuccess) continue;
+        e = cudaMemcpy2DAsync(st.buf[b] + (a - lo) * row, (size_t)row, host + (run.cpu_block + a - run.first) * p.c_block_stride,
+                              (size_t)p.c_block_stride, (size_t)row, (size_t)(z - a), cudaMemcpyHostToDevice,
+                              st.copy_stream);
+      }
+      if (e == cudaSuccess) e = cudaEventRecord(st.copy_done[b], st.copy_stream);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(rk.stream, st.copy_done[b], 0);
+      KvCopyParams q = p;          // the buffer plays the host side: [pair][kv][chunk] of this layer
+      q.cpu_base = reinterpret_cast<uint64_t>(st.buf[b]);
+      q.c_layer_stride = q.c_off = 0;
+      q.c_kv_stride = p.chunk_bytes;
+      q.c_block_stride = row;
+      q.cpu_num_blocks = st.blocks;
+      q.gpu_blocks = gpu_ids + lo;
+      q.num_pairs = (int32_t)(hi - lo);
+      if (hi == j.n) {             // the layer's last launch publishes it
+        q.done_counter = rk.done_counter;
+        q.dev_flags = rk.dev_flags + (size_t)j.counter * L;
+        q.host_flags = rk.host_flags + (size_t)j.counter * L;
+        q.epoch = j.epoch;
+      }
+      if (e == cudaSuccess) e = launch_kv_copy(q, opt_.group.h2d, rk.stream);
+      if (e == cudaSuccess) e = cudaEventRecord(st.kernel_done[b], rk.stream);
+      if (e == cudaSuccess) st.used[b] = true;
+      b = b + 1 == kCeStageBufs ? 0 : b + 1;
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(ev[l], rk.stream);
+  }
+  return e;
 }
 
 // Multi-group restore of one rank: model layer by model layer, one launch per member; the last
@@ -473,7 +552,16 @@ void LayerwiseGroup::run_job(int r, const Job& j) {
   const int64_t* gpu_ids = j.gpu_blocks;
   const int64_t* cpu_ids = j.cpu_blocks;
   if (err == cudaSuccess) err = stage_ids(rk, j, gpu_ids, cpu_ids);
-  for (int b = 0; b < batches && err == cudaSuccess; ++b) {
+  std::vector<CeHostRun> runs;
+  bool staged = false;
+  if (fused && err == cudaSuccess && j.n > 0) {
+    KvCopyParams p;
+    bool skip = false;
+    fill_kv_params(gpus_[(size_t)r], host_, opt_.group, r, R, gpu_ids, cpu_ids, j.n, true, 0, L, 0, p, skip);
+    staged = plan_staged(rk, j, p, runs);
+    if (staged) err = queue_staged(r, j, gpu_ids, runs);
+  }
+  for (int b = 0; b < batches && !staged && err == cudaSuccess; ++b) {
     const int l0 = b * B, l1 = std::min(L, l0 + B);
     KvCopyParams p;
     bool skip = false;

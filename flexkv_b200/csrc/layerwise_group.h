@@ -154,6 +154,7 @@ class LayerwiseGroup {
     int32_t* status = nullptr;          // mapped, kStatusWords
     std::vector<cudaEvent_t> layer_ev;  // [counters][layers]
     cudaEvent_t ev_begin = nullptr;
+    CeStaging staging;                  // the copy-engine form's (queue_staged); blocks = pairs of one layer
     // result of the last job
     int res_status = 0;
     float res_ms = 0.f;
@@ -169,6 +170,11 @@ class LayerwiseGroup {
   void rank_main(int r);
   void run_job(int r, const Job& j);
   void run_job_members(int r, const Job& j);
+  // Copy-engine form of a restore: a layer's rows of the host blocks come into a staging buffer as 2-D copies, one per
+  // run of consecutive host blocks, and a scatter kernel takes them to the pages and publishes the layer's flag. False
+  // when the job is for the kernels: ids out of range, runs or rows too short, no memory for the buffers.
+  bool plan_staged(Rank& rk, const Job& j, const KvCopyParams& p, std::vector<CeHostRun>& runs);
+  cudaError_t queue_staged(int r, const Job& j, const int64_t* gpu_ids, const std::vector<CeHostRun>& runs);
   cudaError_t stage_ids(Rank& rk, const Job& j, const int64_t*& gpu_ids, const int64_t*& cpu_ids);
   void notify(int rank, int counter, int layer_lo, int layer_hi);
   // failure path of a job: records the status for counter_status(), then publishes the epoch to the flags of
@@ -183,6 +189,7 @@ class LayerwiseGroup {
   std::vector<LayerwiseMemberGroup> mgroups_;            // empty for the uniform form
   std::vector<std::vector<LayerMember>> members_;        // [model layer]
   LayerwiseOptions opt_;
+  bool copy_engines_ = false;       // the engine option leaves the choice between kernels and copy engines to us
   std::vector<std::unique_ptr<Rank>> ranks_;
   std::atomic<bool> stop_{false};
   std::vector<int> eventfds_;       // [counters][ranks][layers]

@@ -263,3 +263,41 @@ def test_layerwise_restore_from_a_packed_host_pool(lpb):
     for l in range(L):
         assert torch.equal(kv[l][:, d].view(torch.int16), want[l].view(torch.int16)), l
     del keep
+
+
+@pytest.mark.parametrize("use_mla", [False, True])
+@pytest.mark.parametrize("n", [97, 600])            # 600 x 64 KiB: more than one staging buffer holds
+def test_layers_through_the_copy_engines_carry_the_same_bytes_and_signals(n, use_mla):
+    """Engine `auto`, host blocks in runs: layer rows by copy engine and a scatter per layer; flags, eventfds and
+    bytes as in the kernel form, over two restores on one counter (buffers are reused)."""
+    shape = KVShape("lc", 5, 1, 512, use_mla=True, tokens_per_block=64) if use_mla else \
+        KVShape("lc", 5, 8, 128, tokens_per_block=16)
+    NB = 2 * n + 16
+    kv, reg, pool, _, xfer = _setup(shape, NB=NB)
+    L, K, chunk = shape.num_layers, shape.kv_dim, reg.chunk_bytes
+    host = dict(base=pool.data_ptr(), layer_stride=K * chunk, kv_stride=chunk, block_stride=L * K * chunk, num_blocks=NB)
+    grp = C.LayerwiseGroup([reg.as_native()], host, dict(num_layers=L, kv_dim=K, chunk_bytes=chunk, max_blocks_per_op=NB,
+                                                         notify_mode="hostfunc", num_counters=2, layers_per_batch=-1,
+                                                         h2d=dict(num_ctas=8, tile_bytes=16384, engine=3)))
+    rng = np.random.default_rng(3)
+    cut = n // 3
+    cpu = np.concatenate([np.arange(n + 3, n + 3 + cut), np.arange(5, 5 + n - cut)]).astype(np.int64)
+    src = rng.permutation(NB)[:n].astype(np.int64)
+    assert xfer.transfer(src, cpu, False, 0, L, 0).status == 0
+    s = torch.from_numpy(src).cuda()
+    want = [(t[s] if use_mla else t[:, s]).clone() for t in kv]
+    fds = [grp.eventfd_of(1, 0, l) for l in range(L)]
+    for _ in range(2):
+        for t in kv:
+            t.zero_()
+        dst = rng.permutation(NB)[:n].astype(np.int64)
+        r = grp.restore(dst, cpu, 1)
+        assert r.status == 0 and [_drain(fd) for fd in fds] == [1] * L
+        assert all(b >= a for a, b in zip(r.layer_done_ms, r.layer_done_ms[1:]))
+        d = torch.from_numpy(dst).cuda()
+        for l in range(L):
+            assert torch.equal(kv[l][d] if use_mla else kv[l][:, d], want[l])
+            assert int((kv[l] != 0).any(-1).sum()) == int((want[l] != 0).any(-1).sum())     # nothing beside the pages
+    bad = dst.copy()
+    bad[3] = NB
+    assert grp.restore(bad, cpu, 1).status == 1
