@@ -383,6 +383,7 @@ PYBIND11_MODULE(_C, m) {
              return t.transfer(g, c, n, h2d, ls, nl, engine);
            }, py::arg("gpu_blocks"), py::arg("cpu_blocks"), py::arg("h2d"), py::arg("layer_start"),
            py::arg("num_layers"), py::arg("engine") = -1)
+      .def("bind_thread", &TransferGroup::bind_thread, py::call_guard<py::gil_scoped_release>())
       .def("transfer_refshape", [](TransferGroup& t, I64Array gb, I64Array cb, bool h2d, int ctas) {
              const int64_t* g = gb.data();
              const int64_t* c = cb.data();

@@ -27,8 +27,6 @@ static void check(cudaError_t e, const char* what) {
   }
 }
 
-static constexpr int kInflight = 4;
-
 TransferGroup::TransferGroup(std::vector<GpuSide> gpus, HostSide host, GroupOptions opt)
     : gpus_(std::move(gpus)), host_(host), opt_(opt) {
   if (gpus_.empty()) throw std::invalid_argument("TransferGroup: no GPUs");
@@ -135,9 +133,80 @@ void TransferGroup::fill_params(int r, const Task& t, KvCopyParams& p, bool& ski
                  t.num_layers, t.rotate, p, skip);
 }
 
+// Queues one op of rank `r` on its stream, with the events and status words of `slot`. Called with the rank's exec_mu.
+TransferGroup::Launched TransferGroup::launch_task(int r, const Task& t, int slot) {
+  Rank& rk = *ranks_[(size_t)r];
+  Launched l;
+  KvCopyParams p;
+  bool skip = false;
+  fill_params(r, t, p, skip);
+  p.status = rk.status + slot * kStatusWords;
+  if (skip) return l;
+  l.launched = true;
+  cudaEventRecord(rk.ev0[slot], rk.stream);
+  if (t.engine == kEngineRefshape) {
+    l.err = launch_kv_copy_refshape(p, t.refshape_ctas, rk.stream);
+  } else {
+    KvCopyLaunch cfg = t.h2d ? opt_.h2d : opt_.d2h;
+    if (t.engine >= 0) cfg.engine = t.engine;
+    bool done = false;
+    if (cfg.engine == kEngineCe || cfg.engine == kEngineAuto) {
+      // the id ring is mapped pinned memory: the same pointers are readable here
+      CeAnalysis a = ce_analyze(p.gpu_blocks, p.cpu_blocks, p.num_pairs, p.gpu_num_blocks, p.cpu_num_blocks);
+      CePath path = ce_choose(a, p, cfg.engine == kEngineCe ? CePolicy{INT64_MAX, 0} : opt_.ce_policy);
+      if (path != CePath::KERNEL) {
+        l.err = ce_copy(p, a, path, rk.stream);
+        for (int b = 0; b < kStatusWords; ++b)
+          if (a.status & (1 << b)) p.status[b] = 1;
+        ce_ops_.fetch_add(1, std::memory_order_relaxed);
+        done = true;
+      } else if (opt_.ce_staging_blocks != 0 && (int)gpus_.size() == 1 &&
+                 ce_host_blocks_abut(p, opt_.num_layers, p.chunk_bytes)) {
+        // scattered GPU pages, host blocks in a row: gather into device staging, one large copy per piece
+        const int64_t min_run = std::max<int64_t>(1, (opt_.ce_policy.min_bytes_per_copy + p.c_block_stride - 1) /
+                                                         p.c_block_stride);
+        int64_t* ids = id_ring_ + (size_t)t.slot * 2 * (size_t)opt_.max_blocks_per_op;   // this rank's alone
+        CeStagePlan plan;
+        if (ce_staging_prepare(rk.staging, std::max<int64_t>(0, opt_.ce_staging_blocks), p.c_block_stride) &&
+            ce_plan_staged(p, ids, ids + opt_.max_blocks_per_op, min_run, rk.staging.blocks, plan)) {
+          KvCopyLaunch kcfg = cfg;
+          kcfg.engine = 0;
+          l.err = ce_copy_staged(
+              p, plan, rk.staging,
+              [&kcfg](const KvCopyParams& q, int64_t, cudaStream_t s) { return launch_kv_copy(q, kcfg, s); },
+              rk.stream);
+          ce_ops_.fetch_add(1, std::memory_order_relaxed);
+          staged_ops_.fetch_add(1, std::memory_order_relaxed);
+          done = true;
+        }
+      }
+    }
+    if (!done) {
+      if (cfg.engine >= kEngineCe) cfg.engine = 0;
+      l.err = launch_kv_copy(p, cfg, rk.stream);
+    }
+  }
+  cudaEventRecord(rk.ev1[slot], rk.stream);
+  return l;
+}
+
+// Waits for what launch_task queued; the op's status bits, or a negative CUDA error.
+int TransferGroup::retire_task(int r, const Launched& l, int slot, float& ms) {
+  Rank& rk = *ranks_[(size_t)r];
+  ms = 0.f;
+  if (!l.launched) return 0;
+  cudaError_t e = l.err;
+  if (e == cudaSuccess) e = cudaEventSynchronize(rk.ev1[slot]);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return -(int)e;
+  }
+  cudaEventElapsedTime(&ms, rk.ev0[slot], rk.ev1[slot]);
+  return collect_status(rk.status + slot * kStatusWords);
+}
+
 void TransferGroup::rank_main(int r) {
   Rank& rk = *ranks_[(size_t)r];
-  cudaEvent_t ev0[kInflight], ev1[kInflight];
   try {
     check(cudaSetDevice(gpus_[(size_t)r].device), "cudaSetDevice");
     int lo = 0, hi = 0;
@@ -145,8 +214,8 @@ void TransferGroup::rank_main(int r) {
     check(cudaStreamCreateWithPriority(&rk.stream, cudaStreamNonBlocking, opt_.high_priority_stream ? hi : lo),
           "cudaStreamCreateWithPriority");
     for (int i = 0; i < kInflight; ++i) {
-      check(cudaEventCreate(&ev0[i]), "cudaEventCreate");
-      check(cudaEventCreate(&ev1[i]), "cudaEventCreate");
+      check(cudaEventCreate(&rk.ev0[i]), "cudaEventCreate");
+      check(cudaEventCreate(&rk.ev1[i]), "cudaEventCreate");
     }
     check(cudaHostAlloc((void**)&rk.status, kInflight * kStatusWords * sizeof(int32_t),
                         cudaHostAllocPortable | cudaHostAllocMapped),
@@ -184,81 +253,17 @@ void TransferGroup::rank_main(int r) {
       }
     }
     // launch everything that is queued, then retire in order: consecutive ops overlap their launch latency
-    int launched[kInflight];
-    cudaError_t lerr[kInflight];
+    std::lock_guard<std::mutex> exec(rk.exec_mu);
+    Launched l[kInflight];
+    for (size_t i = 0; i < batch.size(); ++i) l[i] = launch_task(r, batch[i], (int)i);
     for (size_t i = 0; i < batch.size(); ++i) {
-      const Task& t = batch[i];
-      KvCopyParams p;
-      bool skip = false;
-      fill_params(r, t, p, skip);
-      p.status = rk.status + i * kStatusWords;
-      launched[i] = skip ? 0 : 1;
-      lerr[i] = cudaSuccess;
-      if (skip) continue;
-      cudaEventRecord(ev0[i], rk.stream);
-      if (t.engine == kEngineRefshape) {
-        lerr[i] = launch_kv_copy_refshape(p, t.refshape_ctas, rk.stream);
-      } else {
-        KvCopyLaunch cfg = t.h2d ? opt_.h2d : opt_.d2h;
-        if (t.engine >= 0) cfg.engine = t.engine;
-        bool done = false;
-        if (cfg.engine == kEngineCe || cfg.engine == kEngineAuto) {
-          // the id ring is mapped pinned memory: the same pointers are readable here
-          CeAnalysis a = ce_analyze(p.gpu_blocks, p.cpu_blocks, p.num_pairs, p.gpu_num_blocks, p.cpu_num_blocks);
-          CePath path = ce_choose(a, p, cfg.engine == kEngineCe ? CePolicy{INT64_MAX, 0} : opt_.ce_policy);
-          if (path != CePath::KERNEL) {
-            lerr[i] = ce_copy(p, a, path, rk.stream);
-            for (int b = 0; b < kStatusWords; ++b)
-              if (a.status & (1 << b)) p.status[b] = 1;
-            ce_ops_.fetch_add(1, std::memory_order_relaxed);
-            done = true;
-          } else if (opt_.ce_staging_blocks != 0 && (int)gpus_.size() == 1 &&
-                     ce_host_blocks_abut(p, opt_.num_layers, p.chunk_bytes)) {
-            // scattered GPU pages, host blocks in a row: gather into device staging, one large copy per piece
-            const int64_t min_run = std::max<int64_t>(1, (opt_.ce_policy.min_bytes_per_copy + p.c_block_stride - 1) /
-                                                             p.c_block_stride);
-            int64_t* ids = id_ring_ + (size_t)t.slot * 2 * (size_t)opt_.max_blocks_per_op;   // this rank's alone
-            CeStagePlan plan;
-            if (ce_staging_prepare(rk.staging, std::max<int64_t>(0, opt_.ce_staging_blocks), p.c_block_stride) &&
-                ce_plan_staged(p, ids, ids + opt_.max_blocks_per_op, min_run, rk.staging.blocks, plan)) {
-              KvCopyLaunch kcfg = cfg;
-              kcfg.engine = 0;
-              lerr[i] = ce_copy_staged(
-                  p, plan, rk.staging,
-                  [&kcfg](const KvCopyParams& q, int64_t, cudaStream_t s) { return launch_kv_copy(q, kcfg, s); },
-                  rk.stream);
-              ce_ops_.fetch_add(1, std::memory_order_relaxed);
-              staged_ops_.fetch_add(1, std::memory_order_relaxed);
-              done = true;
-            }
-          }
-        }
-        if (!done) {
-          if (cfg.engine >= kEngineCe) cfg.engine = 0;
-          lerr[i] = launch_kv_copy(p, cfg, rk.stream);
-        }
-      }
-      cudaEventRecord(ev1[i], rk.stream);
-    }
-    for (size_t i = 0; i < batch.size(); ++i) {
-      int status = 0;
       float ms = 0.f;
-      if (launched[i]) {
-        cudaError_t e = lerr[i];
-        if (e == cudaSuccess) e = cudaEventSynchronize(ev1[i]);
-        if (e == cudaSuccess) {
-          cudaEventElapsedTime(&ms, ev0[i], ev1[i]);
-          status = collect_status(rk.status + i * kStatusWords);
-        } else {
-          (void)cudaGetLastError();
-          status = -(int)e;
-        }
-      }
+      const int status = retire_task(r, l[i], (int)i, ms);
       finish(batch[i].ticket, status, ms);
     }
   }
   ce_staging_free(rk.staging);
-  for (int i = 0; i < kInflight; ++i) { cudaEventDestroy(ev0[i]); cudaEventDestroy(ev1[i]); }
+  for (int i = 0; i < kInflight; ++i) { cudaEventDestroy(rk.ev0[i]); cudaEventDestroy(rk.ev1[i]); }
   if (rk.status) cudaFreeHost(rk.status);
   if (rk.stream) cudaStreamDestroy(rk.stream);
 }
@@ -278,8 +283,9 @@ void TransferGroup::finish(uint64_t ticket, int status, float ms) {
   }
 }
 
-uint64_t TransferGroup::submit(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d,
-                               int layer_start, int num_layers, int engine_override) {
+// Takes an id ring slot for the op, copies its ids there and enters it among the pending ones.
+TransferGroup::Task TransferGroup::make_task(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d,
+                                             int layer_start, int num_layers, int engine_override) {
   if (n > opt_.max_blocks_per_op) throw std::invalid_argument("TransferGroup: op exceeds max_blocks_per_op");
   if (layer_start < 0 || num_layers < 0 || layer_start + num_layers > opt_.num_layers)
     throw std::invalid_argument("TransferGroup: layer range out of bounds");
@@ -308,12 +314,42 @@ uint64_t TransferGroup::submit(const int64_t* gpu_blocks, const int64_t* cpu_blo
   t.num_layers = num_layers;
   t.engine = engine_override;
   t.refshape_ctas = 4;
+  return t;
+}
+
+uint64_t TransferGroup::submit(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d,
+                               int layer_start, int num_layers, int engine_override) {
+  const Task t = make_task(gpu_blocks, cpu_blocks, n, h2d, layer_start, num_layers, engine_override);
   for (auto& rk : ranks_) {
     { std::lock_guard<std::mutex> g(rk->mu); rk->q.push_back(t); }
     rk->cv.notify_one();
   }
   return t.ticket;
 }
+
+OpResult TransferGroup::transfer(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d,
+                                 int layer_start, int num_layers, int engine_override) {
+  if (ranks_.size() > 1)
+    return wait(submit(gpu_blocks, cpu_blocks, n, h2d, layer_start, num_layers, engine_override));
+  const Task t = make_task(gpu_blocks, cpu_blocks, n, h2d, layer_start, num_layers, engine_override);
+  Rank& rk = *ranks_[0];
+  int before = -1;
+  if (cudaGetDevice(&before) != cudaSuccess) before = -1;
+  {
+    // behind what the rank's thread has in hand; it takes nothing new meanwhile
+    std::lock_guard<std::mutex> exec(rk.exec_mu);
+    float ms = 0.f;
+    cudaError_t e = before == gpus_[0].device ? cudaSuccess : cudaSetDevice(gpus_[0].device);
+    int status;
+    if (e == cudaSuccess) status = retire_task(0, launch_task(0, t, 0), 0, ms);
+    else status = -(int)e;
+    finish(t.ticket, status, ms);
+  }
+  if (before >= 0 && before != gpus_[0].device) cudaSetDevice(before);
+  return wait(t.ticket);
+}
+
+void TransferGroup::bind_thread() { check(cudaSetDevice(gpus_[0].device), "cudaSetDevice"); }
 
 bool TransferGroup::poll(uint64_t ticket) {
   std::lock_guard<std::mutex> g(mu_);

@@ -86,10 +86,12 @@ class TransferGroup {
                   int num_layers, int engine_override = -1);
   OpResult wait(uint64_t ticket);
   bool poll(uint64_t ticket);
+  // Blocking. With one rank the op is launched and waited for on the calling thread: handing it to the rank's thread
+  // and being woken by it cost a 2 MiB op some 40 us.
   OpResult transfer(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d, int layer_start,
-                    int num_layers, int engine_override = -1) {
-    return wait(submit(gpu_blocks, cpu_blocks, n, h2d, layer_start, num_layers, engine_override));
-  }
+                    int num_layers, int engine_override = -1);
+  // Makes the first rank's device the calling thread's, as a thread that will call transfer() does once.
+  void bind_thread();
   // baseline shape for timing comparisons (4 CTAs x 1024 threads, warp per chunk)
   OpResult transfer_refshape(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d, int num_ctas);
 
@@ -111,14 +113,20 @@ class TransferGroup {
     int refshape_ctas;
     uint64_t rotate;   // op counter for RANK_ROTATE
   };
+  static constexpr int kInflight = 4;   // ops of one rank launched before the first is waited for
+  struct Launched {
+    bool launched = false;
+    cudaError_t err = cudaSuccess;
+  };
   struct Rank {
     std::thread th;
     std::mutex mu;
     std::condition_variable cv;
     std::deque<Task> q;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    int32_t* status = nullptr;  // mapped pinned word
+    std::mutex exec_mu;         // held from the first launch of a batch of ops to the retirement of its last
+    cudaEvent_t ev0[kInflight] = {}, ev1[kInflight] = {};
+    int32_t* status = nullptr;  // mapped pinned words, kStatusWords for each op in flight
     CeStaging staging;          // device staging of the gather + large-copy route
     bool ready = false;
     std::string init_error;
@@ -130,6 +138,10 @@ class TransferGroup {
   };
 
   void rank_main(int r);
+  Task make_task(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d, int layer_start,
+                 int num_layers, int engine_override);
+  Launched launch_task(int r, const Task& t, int slot);
+  int retire_task(int r, const Launched& l, int slot, float& ms);
   void fill_params(int r, const Task& t, KvCopyParams& p, bool& skip) const;
   void finish(uint64_t ticket, int status, float ms);
 

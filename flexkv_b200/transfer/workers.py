@@ -66,7 +66,14 @@ class TransferWorker:
     def submit(self, op: TransferOp) -> None:
         self._q.put(op)
 
+    def warm_thread(self) -> None:
+        """First thing on the worker's thread: what its first op would otherwise wait for."""
+
     def _run(self) -> None:
+        try:
+            self.warm_thread()
+        except Exception as e:  # noqa: BLE001 - the first op meets the same condition and reports it
+            flexkv_logger.warning("%s: %s", self.name, e)
         while True:
             op = self._q.get()
             if op is None:
@@ -164,16 +171,21 @@ class GpuHostWorker(TransferWorker):
         nl = self.group_layers if op.num_layers < 0 else op.num_layers
         max_n = self.max_blocks
         status, ms = 0, 0.0
-        tickets = []
-        for lo in range(0, int(cpu.size), max_n):
-            tickets.append(self.group.submit(gpu[lo:lo + max_n], cpu[lo:lo + max_n], self.h2d, op.layer_start, nl))
-        for t in tickets:
-            r = self.group.wait(t)
+        if 0 < cpu.size <= max_n:
+            results = [self.group.transfer(gpu, cpu, self.h2d, op.layer_start, nl)]
+        else:
+            tickets = [self.group.submit(gpu[lo:lo + max_n], cpu[lo:lo + max_n], self.h2d, op.layer_start, nl)
+                       for lo in range(0, int(cpu.size), max_n)]
+            results = [self.group.wait(t) for t in tickets]
+        for r in results:
             status |= r.status if r.status >= 0 else (1 << 30)
             ms += r.gpu_ms
         ok = status == 0
         return OpOutcome(ok, gpu_ms=ms, num_bytes=int(cpu.size) * self._bytes_per_block,
                          error="" if ok else f"kernel status 0x{status:x}")
+
+    def warm_thread(self) -> None:
+        self.group.bind_thread()
 
     group_layers = 0
     max_blocks = 1 << 16
@@ -364,10 +376,24 @@ class QuantGpuHostWorker(TransferWorker):
         self.num_ctas = int(os.environ.get("FLEXKV_QUANT_NUM_CTA", dflt))
         self._torch = torch
         self.streams = {r.device_id: torch.cuda.Stream(device=r.device_id) for r in self.regs}
-        self.status = {r.device_id: torch.zeros(8, dtype=torch.int32, device=f"cuda:{r.device_id}") for r in self.regs}
+        # Kept between ops, which this worker runs one at a time: pinned id buffers and status words that the kernels
+        # address themselves, and a pair of events per device.
+        self._ids = torch.empty((2, 4096), dtype=torch.int64).pin_memory()
+        self.status = {r.device_id: torch.zeros(8, dtype=torch.int32).pin_memory() for r in self.regs}
+        self._words = {d: t.numpy() for d, t in self.status.items()}
+        self._events = {}
         for r in self.regs:
             with torch.cuda.device(r.device_id):
                 _native.C.codec_load_kernels()
+                self._events[r.device_id] = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
+
+    def warm_thread(self) -> None:
+        for d, (e0, e1) in self._events.items():
+            with self._torch.cuda.device(d):
+                e0.record(self.streams[d])
+                e1.record(self.streams[d])
+                e1.synchronize()
+                e0.elapsed_time(e1)
 
     def close(self) -> None:
         self.strategy.detach()
@@ -380,9 +406,13 @@ class QuantGpuHostWorker(TransferWorker):
             gpu, cpu = op.src_block_ids, op.dst_block_ids
         if gpu.size != cpu.size:
             return OpOutcome(False, error=f"unbound GPU blocks: {gpu.size} vs {cpu.size}")
-        keep, evs, nbytes = [], [], 0
-        g_ids = torch.from_numpy(np.ascontiguousarray(gpu, dtype=np.int64)).pin_memory()
-        c_ids = torch.from_numpy(np.ascontiguousarray(cpu, dtype=np.int64)).pin_memory()
+        n, evs, nbytes = int(cpu.size), [], 0
+        if self._ids.shape[1] < n:
+            self._ids = torch.empty((2, 2 * n), dtype=torch.int64).pin_memory()
+        ids = self._ids.numpy()
+        ids[0, :n], ids[1, :n] = gpu, cpu
+        g_ptr = self._ids.data_ptr()
+        c_ptr = g_ptr + 8 * self._ids.shape[1]
         for i, reg in enumerate(self.regs):
             if self.shared and not self.h2d and i > 0:
                 break
@@ -391,27 +421,31 @@ class QuantGpuHostWorker(TransferWorker):
                           idx_kv_mul=reg.idx_kv_mul, g_layer_stride=reg.layer_stride, g_kv_stride=reg.kv_stride,
                           g_block_stride=reg.block_stride, cpu_base=self.host.base, c_layer_stride=self.layer_stride,
                           c_kv_stride=self.kv_stride, c_block_stride=self.host.block_bytes,
-                          c_off=0 if self.shared else i * self.tp_stride, gpu_blocks_ptr=g_ids.data_ptr(),
-                          cpu_blocks_ptr=c_ids.data_ptr(), num_pairs=int(cpu.size), layer_start=op.layer_start,
+                          c_off=0 if self.shared else i * self.tp_stride, gpu_blocks_ptr=g_ptr,
+                          cpu_blocks_ptr=c_ptr, num_pairs=n, layer_start=op.layer_start,
                           num_layers=nl, kv_dim=reg.kv_dim, chunk_bytes=reg.chunk_bytes,
                           gpu_num_blocks=reg.num_blocks, cpu_num_blocks=self.host.num_blocks,
                           status_ptr=self.status[reg.device_id].data_ptr(), h2d=int(self.h2d))
             st = self.streams[reg.device_id]
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0, e1 = self._events[reg.device_id]
             with torch.cuda.device(reg.device_id):
                 e0.record(st)
-                self.strategy.run(params, i, self.num_ctas, st.cuda_stream)
+                try:
+                    self.strategy.run(params, i, self.num_ctas, st.cuda_stream)
+                except Exception:
+                    st.synchronize()        # what was queued still reads the id buffers
+                    raise
                 e1.record(st)
             evs.append((e0, e1, reg.device_id))
-            nbytes += int(cpu.size) * nl * reg.kv_dim * reg.chunk_bytes
+            nbytes += n * nl * reg.kv_dim * reg.chunk_bytes
         status, ms = 0, 0.0
         for e0, e1, dev in evs:
             e1.synchronize()
             ms = max(ms, e0.elapsed_time(e1))
-            words = self.status[dev].tolist()
-            status |= sum(1 << b for b, w in enumerate(words) if w)
-            if status:
-                self.status[dev].zero_()
+            words = self._words[dev]
+            if words.any():
+                status |= sum(1 << b for b, w in enumerate(words.tolist()) if w)
+                words[:] = 0
         return OpOutcome(status == 0, gpu_ms=ms, num_bytes=nbytes,
                          error="" if status == 0 else f"quant kernel status 0x{status:x}")
 
