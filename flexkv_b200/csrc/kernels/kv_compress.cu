@@ -355,7 +355,7 @@ struct __align__(128) GroupState {
 template <bool COMPRESS, int kInStages>
 __global__ void __launch_bounds__(kThreads * kGroups, 1)
 kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict__ size_table, int layers_total,
-                   int tiles_per_chunk) {
+                   int tiles_per_chunk, int lookahead) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   __shared__ GroupState<COMPRESS, kInStages> gstate[kGroups];
   const int grp = threadIdx.x / kThreads;
@@ -504,13 +504,13 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
 
   if (!COMPRESS) { fetch_sizes(0); group_sync(grp); }
   if (tid == 0)
-    for (int64_t it = 0; it < n_mine && it < kInStages - 1; ++it) issue_load(it);
+    for (int64_t it = 0; it < n_mine && it < lookahead; ++it) issue_load(it);
 
   for (int64_t it = 0; it < n_mine; ++it) {
     const int st = (int)(it % kInStages), ob = (int)(it & 1);
     if (!COMPRESS) {
-      // the prefetch below reaches kInStages-1 tiles ahead: refill the size ring before it crosses into a new epoch
-      const int64_t ahead = it + kInStages - 1;
+      // the prefetch below reaches `lookahead` tiles ahead: refill the size ring before it crosses into a new epoch
+      const int64_t ahead = it + lookahead;
       if (ahead % kEpoch == 0 && ahead > 0 && ahead < n_mine) { group_sync(grp); fetch_sizes(ahead); group_sync(grp); }
     }
     if (tid == 0) {
@@ -524,7 +524,7 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
           signalled = lr;
         }
       }
-      if (it + kInStages - 1 < n_mine) issue_load(it + kInStages - 1);
+      if (it + lookahead < n_mine) issue_load(it + lookahead);
       if (it >= 2) ptx::bulk_wait_read<1>();
     }
     group_sync(grp);
@@ -573,6 +573,7 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
 
 // host reads need several tiles in flight per pipeline to cover the PCIe round trip
 constexpr int kInUnpack = 4, kInPack = 3;
+constexpr int64_t kLinkBytesAhead = 768 << 10;
 constexpr int kSmemUnpack = (int)sizeof(Smem<kInUnpack>) * kGroups + 128;
 constexpr int kSmemPack = (int)sizeof(Smem<kInPack>) * kGroups + 128;
 
@@ -600,12 +601,17 @@ cudaError_t launch_kv_compress_bf16(const KvCopyParams& p, uint32_t* size_table,
   const int ctas = (int)((pipes + kGroups - 1) / kGroups);
   const cudaError_t e = kv_compress_load_kernels();
   if (e != cudaSuccess) return e;
+  // Restores: tiles that a pipeline asks for ahead of the one it unpacks. All pipelines together keep the link busy
+  // with some 0.75 MB asked for; what is beyond that arrives at the end all at once and is unpacked with the link idle.
+  const int64_t per_step = pipes * (int64_t)(kCompressTileSlot * 2 / 3);
+  int lookahead = (int)((kLinkBytesAhead + per_step - 1) / per_step);
+  if (lookahead > kInUnpack - 1) lookahead = kInUnpack - 1;
   if (p.h2d)
     kv_compress_kernel<false, kInUnpack><<<ctas, kThreads * kGroups, kSmemUnpack, stream>>>(p, size_table, layers_total,
-                                                                                            tiles_per_chunk);
+                                                                                            tiles_per_chunk, lookahead);
   else
     kv_compress_kernel<true, kInPack><<<ctas, kThreads * kGroups, kSmemPack, stream>>>(p, size_table, layers_total,
-                                                                                       tiles_per_chunk);
+                                                                                       tiles_per_chunk, kInPack - 1);
   return cudaGetLastError();
 }
 
