@@ -96,10 +96,11 @@ bool plan_rows(const KvCopyParams& p, const uint32_t* sizes, const CeHostRun& pi
   // A copy costs 3.5 us beside its bytes, as much as 190 KB of them: one copy of all tiles where they are of one size
   // and at one pitch, else one for each class.
   constexpr int64_t kCopyCostBytes = 190 << 10;
-  const int64_t layer_slot = p.c_layer_stride;
+  const int64_t layer_slot = p.c_layer_stride, pitch = p.c_kv_stride / tiles;
+  const bool even = tiles == 1 || elems % kCompressTileElems == 0;    // every tile slot of the same size
   int64_t moved;
-  if (elems % kCompressTileElems == 0 && rows * classes * (int64_t)widest - apart < (classes - 1) * kCopyCostBytes) {
-    out.push_back(RowCopy{0, kCompressTileSlot, widest, rows * classes});
+  if (even && rows * classes * (int64_t)widest - apart < (classes - 1) * kCopyCostBytes) {
+    out.push_back(RowCopy{0, pitch, widest, rows * classes});
     moved = rows * classes * (int64_t)widest + kCopyCostBytes;
   } else {
     for (int k = 0; k < classes; ++k)
@@ -108,8 +109,8 @@ bool plan_rows(const KvCopyParams& p, const uint32_t* sizes, const CeHostRun& pi
     moved = apart + classes * kCopyCostBytes;
   }
   // 54.5 GB/s in long copies against the kernel's 51 for the used bytes alone. Below 2 MB (40 us) the difference is
-  // less than what changing to the kernel and back costs. Rows below 4 KiB are slower.
-  return moved < used + std::max<int64_t>(used / 16, 2 << 20) && moved / (rows * classes) >= 4096;
+  // less than what changing to the kernel and back costs.
+  return moved < used + std::max<int64_t>(used / 16, 2 << 20);
 }
 
 }  // namespace
@@ -117,7 +118,8 @@ bool plan_rows(const KvCopyParams& p, const uint32_t* sizes, const CeHostRun& pi
 cudaError_t CodecLink::compress_bf16(const KvCopyParams& p, uint32_t* size_table, int layers_total, int num_ctas,
                                      cudaStream_t stream) {
   CeStagePlan pl;
-  if (!p.h2d || size_table == nullptr || p.chunk_bytes % 2048 != 0 || layers_total != num_layers_ ||
+  // rows of chunks below 4096 values are too short for a copy engine: 48.2 GB/s at 2048 values, the kernel 50.4
+  if (!p.h2d || size_table == nullptr || p.chunk_bytes < 8192 || p.chunk_bytes % 2048 != 0 || layers_total != num_layers_ ||
       !plan(p, kMinRowBytes, kRowRampBytes, pl))
     return launch_kv_compress_bf16(p, size_table, layers_total, num_ctas, stream);
   ++staged_ops_;

@@ -6,37 +6,51 @@
 namespace fkv {
 namespace {
 
-// A CTA runs kGroups independent tile pipelines of kThreads threads each (own stage ring, own scratch, own
-// named barrier): one pipeline keeps a single warp per scheduler and waits out every shared-memory round
-// trip; two per SM overlap each other's latencies, so half as many SMs carry the same link rate.
-constexpr int kThreads = 128;
-constexpr int kGroups = 2;
-constexpr int kWarps = kThreads / 32;
-constexpr int kEpoch = 1024;                                  // tile sizes fetched per batch (decompress)
+// A CTA of 256 threads runs independent tile pipelines of T threads each (own stage ring, own scratch, own barrier):
+// one pipeline per scheduler set would wait out every shared-memory round trip; several per SM overlap each other's
+// latencies, so half as many SMs carry the same link rate. A thread codes 64 values, so a full tile of 8192 takes 128
+// threads. The single, shorter tile of a small chunk (one or two KV heads per rank) takes as many as it has chunks of 64:
+// with 128 threads around it, three quarters of them idle and all barriers paid, tiles of 2048 values moved at
+// 33 / 28 GB/s (pack to / unpack from the host, 40 SMs of a B200); now 52.2 / 50.4, as the link allows.
+constexpr int kCtaThreads = 256;
+template <int T>
+struct Pipe {
+  static constexpr int kWarps = T / 32;
+  static constexpr int kGroups = kCtaThreads / T;
+  static constexpr int kTileElems = T * kCodeChunkVals;
+  static constexpr int kSlot = 2 * kTileElems + 128;
+  static constexpr int kEpoch = 8 * T;                        // tile sizes fetched per batch (decompress)
+  // host reads need several tiles in flight per pipeline to cover the PCIe round trip
+  static constexpr int kInUnpack = T == 128 ? 4 : 3, kInPack = 3;
+};
+static_assert(Pipe<128>::kTileElems == kCompressTileElems && Pipe<128>::kSlot == kCompressTileSlot, "full tile");
 constexpr uint64_t kWaitBudgetNs = 2000000000ull;
 constexpr int kTblBatch = 32;                                 // size-table entries written per bulk store (128 bytes)
 constexpr uint32_t kFull = 0xffffffffu;
 
-template <int IN_STAGES>
+template <int T, int IN_STAGES>
 struct __align__(16) Smem {
-  uint8_t in[IN_STAGES][kCompressTileSlot];
-  uint8_t out[2][kCompressTileSlot];
+  uint8_t in[IN_STAGES][Pipe<T>::kSlot];
+  uint8_t out[2][Pipe<T>::kSlot];
 };
 
-// barrier among the kThreads threads of one pipeline (hardware barrier 1 + group; 0 is __syncthreads')
+// barrier among the T threads of one pipeline (hardware barrier 1 + group; 0 is __syncthreads')
+template <int T>
 __device__ __forceinline__ void group_sync(int grp) {
-  asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(kThreads) : "memory");
+  if (T == 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(T) : "memory");
 }
 
 // Per-tile scratch of the coder (static shared memory).
+template <int T>
 struct Scratch {
-  uint32_t hist[kWarps][256];   // per-warp exponent histograms
+  uint32_t hist[Pipe<T>::kWarps][256];   // per-warp exponent histograms
   uint32_t cnt[256];            // their sum
   uint32_t code[256];           // exponent -> code bits (low 24) | code length (high 8)
   uint8_t nz[256];              // exponents that occur, compacted
   uint8_t rank[256];            // exponent -> frequency rank (kCodeRanks and above: no code of its own)
   uint32_t seg[8];              // occurrences per 32-exponent segment
-  uint32_t warp_tot[kWarps];
+  uint32_t warp_tot[Pipe<T>::kWarps];
   uint32_t cost[2];             // sampled code bits under mode 1 and mode 2
 };
 
@@ -60,7 +74,9 @@ __device__ __forceinline__ uint32_t code_of(int mode, int r, int e) {
 }
 __device__ __forceinline__ uint32_t code_len(int mode, int r) { return code_of(mode, r, 0) >> 24; }
 
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, Scratch& sc, uint32_t& total, int grp) {
+template <int T>
+__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, Scratch<T>& sc, uint32_t& total, int grp) {
+  constexpr int kWarps = Pipe<T>::kWarps;
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & (kWarps - 1);
   uint32_t incl = v;
 #pragma unroll
@@ -69,7 +85,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, Scratch& sc
     if (lane >= o) incl += u;
   }
   if (lane == 31) sc.warp_tot[warp] = incl;
-  group_sync(grp);
+  group_sync<T>(grp);
   uint32_t base = 0;
   total = 0;
 #pragma unroll
@@ -82,14 +98,17 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, Scratch& sc
 }
 
 // Packs `elems` bf16 values at `in` into `out`; every thread returns the packed size (a multiple of 16).
-__device__ uint32_t compress_tile(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, int elems, Scratch& sc,
+template <int T>
+__device__ uint32_t compress_tile(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, int elems, Scratch<T>& sc,
                                   int grp) {
-  const int tid = threadIdx.x & (kThreads - 1), lane = tid & 31, warp = tid >> 5;
+  constexpr int kWarps = Pipe<T>::kWarps;
+  constexpr int kBins = 256 / T;             // exponents per thread: tid, tid + T, ...
+  const int tid = threadIdx.x & (T - 1), lane = tid & 31, warp = tid >> 5;
   const int n_chunks = elems / kCodeChunkVals;
   const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
   const int off_sm = kCodeHeaderBytes + n_chunks, off_exp = off_sm + elems;
   constexpr int W = kCodeChunkVals / 2;     // words per chunk
-  for (int i = tid; i < kWarps * 256; i += kThreads) (&sc.hist[0][0])[i] = 0;
+  for (int i = tid; i < kWarps * 256; i += T) (&sc.hist[0][0])[i] = 0;
   if (tid < kCodeRanks) out[16 + tid] = 0;
   if (tid < 2) sc.cost[tid] = 0;
   // this thread's chunk stays in registers for the three passes over it
@@ -102,7 +121,7 @@ __device__ uint32_t compress_tile(const uint8_t* __restrict__ in, uint8_t* __res
 #pragma unroll
     for (int k = 0; k < W; ++k) x[k] = 0;
   }
-  group_sync(grp);
+  group_sync<T>(grp);
   // 1: exponent histogram over a sample (the first kCodeSampleWords words of every chunk: ranks only steer
   //    the code lengths, any table decodes) and the sign|mantissa plane
   if (active) {
@@ -117,30 +136,36 @@ __device__ uint32_t compress_tile(const uint8_t* __restrict__ in, uint8_t* __res
                                             ((((x[k] >> 24) & 0x80u) | ((x[k] >> 16) & 0x7fu)) << 8));
     }
   }
-  group_sync(grp);
+  group_sync<T>(grp);
   // 2: counts, the exponents that occur, their frequency ranks -> code table and symbol table
-  uint32_t c0 = 0, c1 = 0;
+  uint32_t cb[kBins], occ[kBins];
 #pragma unroll
-  for (int w = 0; w < kWarps; ++w) { c0 += sc.hist[w][tid]; c1 += sc.hist[w][tid + 128]; }
-  sc.cnt[tid] = c0;
-  sc.cnt[tid + 128] = c1;
-  sc.rank[tid] = 255;
-  sc.rank[tid + 128] = 255;
-  const uint32_t b0 = __ballot_sync(kFull, c0 > 0), b1 = __ballot_sync(kFull, c1 > 0);
-  if (lane == 0) { sc.seg[warp] = __popc(b0); sc.seg[4 + warp] = __popc(b1); }
-  group_sync(grp);
-  uint32_t base0 = 0, base1 = 0, n_nz = 0;
+  for (int j = 0; j < kBins; ++j) {
+    const int e = tid + j * T;
+    uint32_t c = 0;
 #pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    const uint32_t v = sc.seg[s];
-    if (s < warp) base0 += v;
-    if (s < 4 + warp) base1 += v;
+    for (int w = 0; w < kWarps; ++w) c += sc.hist[w][e];
+    cb[j] = c;
+    sc.cnt[e] = c;
+    sc.rank[e] = 255;
+    occ[j] = __ballot_sync(kFull, c > 0);
+    if (lane == 0) sc.seg[warp + j * kWarps] = __popc(occ[j]);
+  }
+  group_sync<T>(grp);
+  uint32_t n_nz = 0, at[kBins] = {};
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    const uint32_t v = sc.seg[g];
+#pragma unroll
+    for (int j = 0; j < kBins; ++j)
+      if (g < warp + j * kWarps) at[j] += v;
     n_nz += v;
   }
   const uint32_t lt = (1u << lane) - 1u;
-  if (c0 > 0) sc.nz[base0 + __popc(b0 & lt)] = (uint8_t)tid;
-  if (c1 > 0) sc.nz[base1 + __popc(b1 & lt)] = (uint8_t)(tid + 128);
-  group_sync(grp);
+#pragma unroll
+  for (int j = 0; j < kBins; ++j)
+    if (cb[j] > 0) sc.nz[at[j] + __popc(occ[j] & lt)] = (uint8_t)(tid + j * T);
+  group_sync<T>(grp);
   if (n_nz <= 32) {
     // the usual case: one warp ranks all occurring exponents through shuffles
     if (warp == 0) {
@@ -166,10 +191,10 @@ __device__ uint32_t compress_tile(const uint8_t* __restrict__ in, uint8_t* __res
       if (lane == 0) { sc.cost[0] = a1; sc.cost[1] = a2; }
     }
   } else {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t c = h ? c1 : c0;
-      const int b = tid + 128 * h;
+#pragma unroll 1
+    for (int j = 0; j < kBins; ++j) {
+      const int b = tid + j * T;
+      const uint32_t c = sc.cnt[b];
       if (c == 0) continue;
       int r = 0;
       for (uint32_t i = 0; i < n_nz; ++i) {
@@ -183,15 +208,17 @@ __device__ uint32_t compress_tile(const uint8_t* __restrict__ in, uint8_t* __res
       atomicAdd(&sc.cost[1], c * code_len(2, r < kCodeRanks ? r : kCodeRanks));
     }
   }
-  group_sync(grp);
+  group_sync<T>(grp);
   // the code shape that is shorter for the sample; every exponent's code under it
   const int mode = sc.cost[1] < sc.cost[0] ? 2 : 1;
   {
-    const int r0 = sc.rank[tid], r1 = sc.rank[tid + 128];
-    sc.code[tid] = code_of(mode, r0 < kCodeRanks ? r0 : kCodeRanks, tid);
-    sc.code[tid + 128] = code_of(mode, r1 < kCodeRanks ? r1 : kCodeRanks, tid + 128);
+#pragma unroll
+    for (int j = 0; j < kBins; ++j) {
+      const int e = tid + j * T, r = sc.rank[e];
+      sc.code[e] = code_of(mode, r < kCodeRanks ? r : kCodeRanks, e);
+    }
   }
-  group_sync(grp);
+  group_sync<T>(grp);
   // 3: coded size of every chunk, their offsets, and whether coding pays at all
   uint32_t bits = 0;
   if (active) {
@@ -202,7 +229,7 @@ __device__ uint32_t compress_tile(const uint8_t* __restrict__ in, uint8_t* __res
   }
   const uint32_t nbytes = (bits + 7) >> 3;
   uint32_t total_exp;
-  const uint32_t myoff = block_exclusive_scan(nbytes, sc, total_exp, grp);
+  const uint32_t myoff = block_exclusive_scan<T>(nbytes, sc, total_exp, grp);
   const uint32_t coded_total = ((uint32_t)off_exp + total_exp + 15u) & ~15u;
   const uint32_t raw_total = 16u + (uint32_t)elems * 2u;
   const bool coded = coded_total < raw_total;
@@ -244,7 +271,7 @@ __device__ uint32_t compress_tile(const uint8_t* __restrict__ in, uint8_t* __res
   // 4b: exponents too spread out for the code to pay: the tile travels raw behind its header
   const uint4* src = reinterpret_cast<const uint4*>(in);
   uint4* dstv = reinterpret_cast<uint4*>(out + 16);
-  for (int i = tid; i < elems / 8; i += kThreads) dstv[i] = src[i];
+  for (int i = tid; i < elems / 8; i += T) dstv[i] = src[i];
   if (tid == 0) {
     out[0] = 0;
     out[1] = 0;
@@ -258,9 +285,10 @@ __device__ uint32_t compress_tile(const uint8_t* __restrict__ in, uint8_t* __res
 
 // Unpacks a tile of `size` bytes at `in` into `elems` bf16 values at `out`. False (for every thread) when the
 // header or the chunk table does not describe a tile of this shape and size; nothing past the slot is read.
+template <int T>
 __device__ bool decompress_tile(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, int elems, uint32_t size,
-                                Scratch& sc, int grp) {
-  const int tid = threadIdx.x & (kThreads - 1);
+                                Scratch<T>& sc, int grp) {
+  const int tid = threadIdx.x & (T - 1);
   const int mode = in[0];
   const uint32_t total = *reinterpret_cast<const uint32_t*>(in + 4);
   const uint32_t elems_h = *reinterpret_cast<const uint32_t*>(in + 8);
@@ -269,7 +297,7 @@ __device__ bool decompress_tile(const uint8_t* __restrict__ in, uint8_t* __restr
     if (size != 16u + (uint32_t)elems * 2u) return false;
     const uint4* src = reinterpret_cast<const uint4*>(in + 16);
     uint4* dst = reinterpret_cast<uint4*>(out);
-    for (int i = tid; i < elems / 8; i += kThreads) dst[i] = src[i];
+    for (int i = tid; i < elems / 8; i += T) dst[i] = src[i];
     return true;
   }
   const int n_chunks = elems / kCodeChunkVals;
@@ -277,7 +305,7 @@ __device__ bool decompress_tile(const uint8_t* __restrict__ in, uint8_t* __restr
   const int off_sm = kCodeHeaderBytes + n_chunks, off_exp = off_sm + elems;
   const uint32_t nbytes = tid < n_chunks ? in[kCodeHeaderBytes + tid] : 0u;
   uint32_t total_exp;
-  const uint32_t myoff = block_exclusive_scan(nbytes, sc, total_exp, grp);
+  const uint32_t myoff = block_exclusive_scan<T>(nbytes, sc, total_exp, grp);
   if ((uint32_t)off_exp + total_exp > size) return false;       // same value in every thread
   if (tid < n_chunks) {
     const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
@@ -339,7 +367,7 @@ __device__ bool decompress_tile(const uint8_t* __restrict__ in, uint8_t* __restr
 }
 
 // static shared state of one pipeline
-template <bool COMPRESS, int IN_STAGES>
+template <bool COMPRESS, int T, int IN_STAGES>
 struct __align__(128) GroupState {
   uint32_t tbl[3][kTblBatch];
   uint64_t full[IN_STAGES];
@@ -347,21 +375,23 @@ struct __align__(128) GroupState {
   uint64_t table_idx[IN_STAGES];
   int32_t elems[IN_STAGES];
   uint32_t in_bytes[IN_STAGES];
-  uint32_t sizes[COMPRESS ? 1 : kEpoch];
-  Scratch sc;
+  uint32_t sizes[COMPRESS ? 1 : Pipe<T>::kEpoch];
+  Scratch<T> sc;
   int abort;
 };
 
-template <bool COMPRESS, int kInStages>
-__global__ void __launch_bounds__(kThreads * kGroups, 1)
+template <bool COMPRESS, int T>
+__global__ void __launch_bounds__(kCtaThreads, 1)
 kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict__ size_table, int layers_total,
                    int tiles_per_chunk, int lookahead) {
+  constexpr int kInStages = COMPRESS ? Pipe<T>::kInPack : Pipe<T>::kInUnpack;
+  constexpr int kGroups = Pipe<T>::kGroups, kEpoch = Pipe<T>::kEpoch;
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  __shared__ GroupState<COMPRESS, kInStages> gstate[kGroups];
-  const int grp = threadIdx.x / kThreads;
-  const int tid = threadIdx.x % kThreads;
-  Smem<kInStages>& sm = reinterpret_cast<Smem<kInStages>*>(smem_raw)[grp];
-  GroupState<COMPRESS, kInStages>& gs = gstate[grp];
+  __shared__ GroupState<COMPRESS, T, kInStages> gstate[kGroups];
+  const int grp = threadIdx.x / T;
+  const int tid = threadIdx.x % T;
+  Smem<T, kInStages>& sm = reinterpret_cast<Smem<T, kInStages>*>(smem_raw)[grp];
+  GroupState<COMPRESS, T, kInStages>& gs = gstate[grp];
   uint64_t* full = gs.full;
   uint64_t* s_dst = gs.dst;
   uint64_t* s_table_idx = gs.table_idx;
@@ -369,7 +399,7 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
   int32_t* s_elems = gs.elems;
   uint32_t* s_in_bytes = gs.in_bytes;
   uint32_t* s_sizes = gs.sizes;
-  Scratch& sc = gs.sc;
+  Scratch<T>& sc = gs.sc;
   int& s_abort = gs.abort;
   // every pipeline is a CTA of its own as far as the work split and the completion count go
   const int64_t vcta = (int64_t)blockIdx.x * kGroups + grp, vgrid = (int64_t)gridDim.x * kGroups;
@@ -379,7 +409,7 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
     s_abort = 0;
     ptx::fence_mbar_init();
   }
-  group_sync(grp);
+  group_sync<T>(grp);
 
   const int64_t chunk_elems = p.chunk_bytes / 2;
   const bool by_layer = !COMPRESS && p.layer_major;
@@ -476,7 +506,7 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
 
   // decompress: the sizes of this CTA's next kEpoch tiles are fetched by all threads at once
   auto fetch_sizes = [&](int64_t from) {
-    for (int64_t it = from + tid; it < n_mine && it < from + kEpoch; it += kThreads) {
+    for (int64_t it = from + tid; it < n_mine && it < from + kEpoch; it += T) {
       uint64_t g, c, tidx;
       int32_t elems;
       int keep = err;
@@ -502,7 +532,7 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
     tbl_n = 0;
   };
 
-  if (!COMPRESS) { fetch_sizes(0); group_sync(grp); }
+  if (!COMPRESS) { fetch_sizes(0); group_sync<T>(grp); }
   if (tid == 0)
     for (int64_t it = 0; it < n_mine && it < lookahead; ++it) issue_load(it);
 
@@ -511,7 +541,7 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
     if (!COMPRESS) {
       // the prefetch below reaches `lookahead` tiles ahead: refill the size ring before it crosses into a new epoch
       const int64_t ahead = it + lookahead;
-      if (ahead % kEpoch == 0 && ahead > 0 && ahead < n_mine) { group_sync(grp); fetch_sizes(ahead); group_sync(grp); }
+      if (ahead % kEpoch == 0 && ahead > 0 && ahead < n_mine) { group_sync<T>(grp); fetch_sizes(ahead); group_sync<T>(grp); }
     }
     if (tid == 0) {
       if (by_layer && p.done_counter) {
@@ -527,24 +557,24 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
       if (it + lookahead < n_mine) issue_load(it + lookahead);
       if (it >= 2) ptx::bulk_wait_read<1>();
     }
-    group_sync(grp);
+    group_sync<T>(grp);
     const int ok = ptx::mbar_wait_bounded(&full[st], (phases >> st) & 1u, kWaitBudgetNs) ? 1 : 0;
     phases ^= 1u << st;
     if (!ok) s_abort = 1;                 // any thread whose wait ran out; the pipeline leaves together
-    group_sync(grp);
+    group_sync<T>(grp);
     if (*reinterpret_cast<volatile int*>(&s_abort)) break;
     const int elems = s_elems[st];
     uint32_t out_bytes = 0;
     if (elems > 0) {
       if (COMPRESS) {
-        out_bytes = compress_tile(sm.in[st], sm.out[ob], elems, sc, grp);
+        out_bytes = compress_tile<T>(sm.in[st], sm.out[ob], elems, sc, grp);
       } else {
-        if (decompress_tile(sm.in[st], sm.out[ob], elems, s_in_bytes[st], sc, grp)) out_bytes = (uint32_t)elems * 2;
+        if (decompress_tile<T>(sm.in[st], sm.out[ob], elems, s_in_bytes[st], sc, grp)) out_bytes = (uint32_t)elems * 2;
         else err |= KV_ERR_PAYLOAD_OVERFLOW;   // same verdict in every thread; thread 0 reports it
       }
     }
     ptx::fence_proxy_async_smem();
-    group_sync(grp);
+    group_sync<T>(grp);
     if (tid == 0) {
       if (out_bytes > 0) {
         ptx::bulk_s2g(reinterpret_cast<void*>(s_dst[st]), sm.out[ob], out_bytes);
@@ -571,19 +601,52 @@ kv_compress_kernel(const __grid_constant__ KvCopyParams p, uint32_t* __restrict_
   }
 }
 
-// host reads need several tiles in flight per pipeline to cover the PCIe round trip
-constexpr int kInUnpack = 4, kInPack = 3;
 constexpr int64_t kLinkBytesAhead = 768 << 10;
-constexpr int kSmemUnpack = (int)sizeof(Smem<kInUnpack>) * kGroups + 128;
-constexpr int kSmemPack = (int)sizeof(Smem<kInPack>) * kGroups + 128;
+
+template <bool COMPRESS, int T>
+constexpr int pipe_smem() {
+  return (int)sizeof(Smem<T, COMPRESS ? Pipe<T>::kInPack : Pipe<T>::kInUnpack>) * Pipe<T>::kGroups;
+}
+
+template <bool COMPRESS, int T>
+cudaError_t load_pipe() {
+  return cudaFuncSetAttribute(kv_compress_kernel<COMPRESS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              pipe_smem<COMPRESS, T>());
+}
+
+// `sms` CTAs at most, fewer when there are not that many tiles.
+template <bool COMPRESS, int T>
+cudaError_t launch_pipe(const KvCopyParams& p, uint32_t* size_table, int layers_total, int tiles_per_chunk,
+                        int64_t total, int64_t sms, cudaStream_t stream) {
+  const cudaError_t e = load_pipe<COMPRESS, T>();
+  if (e != cudaSuccess) return e;
+  constexpr int G = Pipe<T>::kGroups;
+  const int64_t ctas = sms < (total + G - 1) / G ? sms : (total + G - 1) / G;
+  int lookahead = Pipe<T>::kInPack - 1;
+  if (!COMPRESS) {
+    // Tiles that a pipeline asks for ahead of the one it unpacks. All pipelines together keep the link busy with some
+    // 0.75 MB asked for; what is beyond that arrives at the end all at once and is unpacked with the link idle, and
+    // on some hosts reads are slower the more of them there are. B200, before (three tiles each) -> now: 11 blocks of
+    // llama3-8b 369 -> 356 us, 56 of deepseek-v3 3739 -> 3530 us.
+    const int64_t per_step = ctas * G * (Pipe<T>::kSlot * 2 / 3);
+    const int64_t want = (kLinkBytesAhead + per_step - 1) / per_step;
+    lookahead = (int)(want < Pipe<T>::kInUnpack - 1 ? want : Pipe<T>::kInUnpack - 1);
+  }
+  kv_compress_kernel<COMPRESS, T><<<(unsigned)ctas, kCtaThreads, pipe_smem<COMPRESS, T>(), stream>>>(
+      p, size_table, layers_total, tiles_per_chunk, lookahead);
+  return cudaGetLastError();
+}
 
 }  // namespace
 
 cudaError_t kv_compress_load_kernels() {
-  const cudaError_t e = cudaFuncSetAttribute(kv_compress_kernel<false, kInUnpack>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemUnpack);
-  return e != cudaSuccess ? e : cudaFuncSetAttribute(kv_compress_kernel<true, kInPack>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPack);
+  cudaError_t e = load_pipe<false, 128>();
+  if (e == cudaSuccess) e = load_pipe<true, 128>();
+  if (e == cudaSuccess) e = load_pipe<false, 64>();
+  if (e == cudaSuccess) e = load_pipe<true, 64>();
+  if (e == cudaSuccess) e = load_pipe<false, 32>();
+  if (e == cudaSuccess) e = load_pipe<true, 32>();
+  return e;
 }
 
 cudaError_t launch_kv_compress_bf16(const KvCopyParams& p, uint32_t* size_table, int layers_total, int num_ctas,
@@ -596,23 +659,13 @@ cudaError_t launch_kv_compress_bf16(const KvCopyParams& p, uint32_t* size_table,
   const int tiles_per_chunk = (int)compress_tiles_per_chunk(chunk_elems);
   const int64_t total = (int64_t)p.num_pairs * p.num_layers * p.kv_dim * tiles_per_chunk;
   // `num_ctas` counts 128-thread tile pipelines; two of them share a CTA (and an SM)
-  int64_t pipes = num_ctas > 0 ? num_ctas : 32;
-  if (pipes > total) pipes = total;
-  const int ctas = (int)((pipes + kGroups - 1) / kGroups);
-  const cudaError_t e = kv_compress_load_kernels();
-  if (e != cudaSuccess) return e;
-  // Restores: tiles that a pipeline asks for ahead of the one it unpacks. All pipelines together keep the link busy
-  // with some 0.75 MB asked for; what is beyond that arrives at the end all at once and is unpacked with the link idle.
-  const int64_t per_step = pipes * (int64_t)(kCompressTileSlot * 2 / 3);
-  int lookahead = (int)((kLinkBytesAhead + per_step - 1) / per_step);
-  if (lookahead > kInUnpack - 1) lookahead = kInUnpack - 1;
-  if (p.h2d)
-    kv_compress_kernel<false, kInUnpack><<<ctas, kThreads * kGroups, kSmemUnpack, stream>>>(p, size_table, layers_total,
-                                                                                            tiles_per_chunk, lookahead);
-  else
-    kv_compress_kernel<true, kInPack><<<ctas, kThreads * kGroups, kSmemPack, stream>>>(p, size_table, layers_total,
-                                                                                       tiles_per_chunk, kInPack - 1);
-  return cudaGetLastError();
+  const int64_t sms = ((num_ctas > 0 ? num_ctas : 32) + 1) / 2;
+  auto go = [&](auto pack, auto unpack) {
+    return (p.h2d ? unpack : pack)(p, size_table, layers_total, tiles_per_chunk, total, sms, stream);
+  };
+  if (chunk_elems <= Pipe<32>::kTileElems) return go(launch_pipe<true, 32>, launch_pipe<false, 32>);
+  if (chunk_elems <= Pipe<64>::kTileElems) return go(launch_pipe<true, 64>, launch_pipe<false, 64>);
+  return go(launch_pipe<true, 128>, launch_pipe<false, 128>);
 }
 
 }  // namespace fkv

@@ -153,7 +153,7 @@ def test_kvmanager_with_lossless_codec_host_and_ssd(tmp_path):
 @pytest.mark.parametrize("shape,spread", [(KVShape("r1", 16, 8, 128, tokens_per_block=16), False),   # two full tiles a chunk
                                           (KVShape("r1", 16, 8, 128, tokens_per_block=16), True),    # some tiles raw
                                           (KVShape("r2", 15, 1, 576, use_mla=True, tokens_per_block=64), False),
-                                          (KVShape("r3", 48, 1, 128, tokens_per_block=16), False)])  # 3 KiB rows
+                                          (KVShape("r3", 48, 1, 256, tokens_per_block=16), False)])  # 6 KiB rows, one tile a chunk
 def test_restore_through_the_copy_engines_matches_the_kernel(shape, spread):
     """Host runs come in as rows of the used bytes, stray blocks by the kernel; a piece whose tiles differ much in
     size stays with the kernel. Tiles beyond the used bytes are never looked at: the slots hold garbage there."""
@@ -202,3 +202,45 @@ def test_restore_through_the_copy_engines_matches_the_kernel(shape, spread):
                        torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     assert decode_status(status) == 16
+
+
+@pytest.mark.parametrize("elems", [1024, 2048, 3072, 4096, 5120])     # 32, 32, 64, 64 and 128 threads per tile
+@pytest.mark.parametrize("ctas", [2, 80])
+def test_small_chunks_pack_to_the_reference_bytes_and_back(elems, ctas):
+    """A chunk of one short tile takes as many threads as it has 64-value pieces; scattered and wild exponents too."""
+    dev = torch.device("cuda:0")
+    shape = KVShape("s", 3, 1, elems // 8, tokens_per_block=8)
+    NB, n = 80, 61
+    kv, layout = alloc_paged_cache(shape, NB, dev, "vllm", fill="normal", seed=9)
+    kv[1][0].mul_(torch.exp(3 * torch.randn(shape.head_size, device=dev)))            # more than 16 exponents: escapes
+    kv[1][1, :NB // 2].view(torch.int16).random_(-32768, 32767)                       # more than 32 exponents, raw tiles
+    kv[2][0].zero_()
+    reg = register_tensors(kv, layout)
+    E = reg.chunk_bytes // 2
+    assert E == elems
+    slot = chunk_slot_bytes(E)
+    L, K = shape.num_layers, shape.kv_dim
+    pool = torch.zeros(NB, L, K, slot, dtype=torch.uint8).pin_memory()
+    table = torch.zeros(size_table_entries(NB, L, K, E), dtype=torch.int32).pin_memory()
+    host = HostSide(pool.data_ptr(), K * slot, slot, L * K * slot, NB)
+    rng = np.random.default_rng(2)
+    g, c, g2 = (rng.permutation(NB)[:n].astype(np.int64) for _ in range(3))
+    status = new_status(dev)
+    keep = kv_compress(reg, host, table, g, c, h2d=False, num_ctas=ctas, status=status)
+    torch.cuda.synchronize()
+    sizes = table.view(NB, L, K)
+    saved = [t.clone() for t in kv]
+    for i in rng.permutation(n)[:9]:
+        for l in range(L):
+            for k in range(K):
+                want = reference_compress_tile(saved[l][k, int(g[i])].reshape(-1).cpu())
+                assert int(sizes[c[i], l, k]) == want.numel()
+                assert torch.equal(pool[int(c[i]), l, k, :want.numel()], want)
+    for t in kv:
+        t.zero_()
+    keep += kv_compress(reg, host, table, g2, c, h2d=True, num_ctas=ctas, status=status)
+    torch.cuda.synchronize()
+    assert decode_status(status) == 0
+    a, b = torch.from_numpy(g).to(dev), torch.from_numpy(g2).to(dev)
+    for t, s in zip(kv, saved):
+        assert torch.equal(t[:, b].view(torch.int16), s[:, a].view(torch.int16))
