@@ -8,18 +8,25 @@
 namespace fkv {
 namespace {
 
-// One tile pipeline of 256 threads per CTA, two CTAs to an SM. Against the host the link bounds it. Within HBM (packing
-// into the staging buffer of the copy-engine route) the latency of the arithmetic does. Eight lanes hold a group, 16
-// values each, so that four groups share a warp and a maximum takes three shuffles instead of five. Packing within HBM,
-// GB/s of bf16 on B200, 48 / 148 CTAs: a warp per group 144 / 438 (128 threads), eight lanes per group 226 / 680, 256
-// threads and quant2 below 371 / 1097; unpacking 504 / 1481 -> 685 / 1973.
-constexpr int kThreads = 256;
-constexpr int kTileElems = 8192;             // 16 KiB of bf16 in, 8 KiB + 256 B out
+// A CTA of 256 threads runs tile pipelines of T threads each, two CTAs to an SM. Against the host the link bounds it.
+// Within HBM (packing into the staging buffer of the copy-engine route) the latency of the arithmetic does. Eight lanes
+// hold a group, 16 values each, so that four groups share a warp and a maximum takes three shuffles instead of five.
+// Packing within HBM, GB/s of bf16 on B200, 48 / 148 CTAs: a warp per group 144 / 438 (128 threads), eight lanes per
+// group 226 / 680, 256 threads and quant2 below 371 / 1097; unpacking 504 / 1481 -> 685 / 1973. The short tile of a
+// small chunk (one or two KV heads per rank) takes 32 values per thread as a full one does, in a pipeline of its own.
+constexpr int kCtaThreads = 256;
 constexpr int kLanesPerGroup = 8;
 constexpr uint64_t kWaitBudgetNs = 2000000000ull;
 
-template <bool PACK>
+template <int T>
+struct Pipe {
+  static constexpr int kTileElems = 32 * T;  // T = 256: 16 KiB of bf16 in, 8 KiB + 256 B out
+  static constexpr int kGroups = kCtaThreads / T;
+};
+
+template <bool PACK, int T>
 struct __align__(16) Smem {
+  static constexpr int kTileElems = Pipe<T>::kTileElems;
   // host reads need more tiles in flight than HBM reads
   static constexpr int kInStages = PACK ? 4 : 6;
   // pack: in = bf16 tile; unpack: in = e4m3 payload followed by its scales
@@ -27,6 +34,12 @@ struct __align__(16) Smem {
   uint8_t out[2][kTileElems * 2];
   float out_scales[2][kTileElems / kQuantGroup];
 };
+
+// barrier among the threads of one pipeline (hardware barrier 1 + pipeline; 0 is __syncthreads')
+template <int T>
+__device__ __forceinline__ void pipe_sync(int pipe) {
+  asm volatile("bar.sync %0, %1;" ::"r"(pipe + 1), "n"(T) : "memory");
+}
 
 // largest value among the lanes that hold a group
 __device__ __forceinline__ float group_max(float v) {
@@ -67,34 +80,43 @@ __device__ __forceinline__ uint32_t dequant2(uint32_t q, float scale) {
   return *reinterpret_cast<uint32_t*>(&o);
 }
 
-template <bool PACK>
-__global__ void __launch_bounds__(kThreads, 2) kv_quant_fp8_kernel(const __grid_constant__ KvCopyParams p,
-                                                                   int tiles_per_chunk) {
-  constexpr int kInStages = Smem<PACK>::kInStages;
+template <bool PACK, int T>
+__global__ void __launch_bounds__(kCtaThreads, 2) kv_quant_fp8_kernel(const __grid_constant__ KvCopyParams p,
+                                                                      int tiles_per_chunk) {
+  constexpr int kInStages = Smem<PACK, T>::kInStages, kTileElems = Pipe<T>::kTileElems, kGroups = Pipe<T>::kGroups;
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  Smem<PACK>& sm = *reinterpret_cast<Smem<PACK>*>(smem_raw);
-  __shared__ __align__(8) uint64_t full[kInStages];
-  __shared__ uint64_t s_dst[kInStages];       // destination of the tile's payload
-  __shared__ uint64_t s_dst2[kInStages];      // pack: destination of the tile's scales
-  __shared__ int32_t s_elems[kInStages];      // 0 = skipped tile
-  __shared__ int s_abort;
+  struct State {
+    uint64_t full[kInStages];
+    uint64_t dst[kInStages];       // destination of the tile's payload
+    uint64_t dst2[kInStages];      // pack: destination of the tile's scales
+    int32_t elems[kInStages];      // 0 = skipped tile
+    int abort;
+  };
+  __shared__ __align__(8) State state[kGroups];
+  const int pipe = threadIdx.x / T, tid = threadIdx.x % T, warp = tid >> 5, lane = tid & 31;
+  Smem<PACK, T>& sm = reinterpret_cast<Smem<PACK, T>*>(smem_raw)[pipe];
+  uint64_t* const full = state[pipe].full;
+  uint64_t* const s_dst = state[pipe].dst;
+  uint64_t* const s_dst2 = state[pipe].dst2;
+  int32_t* const s_elems = state[pipe].elems;
+  int& s_abort = state[pipe].abort;
+  const int64_t vcta = (int64_t)blockIdx.x * kGroups + pipe, vgrid = (int64_t)gridDim.x * kGroups;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < kInStages; ++s) ptx::mbar_init(&full[s], 1);
     s_abort = 0;
     ptx::fence_mbar_init();
   }
-  __syncthreads();
+  pipe_sync<T>(pipe);
 
   const int64_t chunk_elems = p.chunk_bytes / 2;
   const int32_t span = p.num_layers * p.kv_dim * tiles_per_chunk;
   const int64_t total = (int64_t)span * p.num_pairs;
-  // every CTA owns one contiguous run of tiles: consecutive tiles share their block ids (fetched
+  // every pipeline owns one contiguous run of tiles: consecutive tiles share their block ids (fetched
   // once per pair, possibly over PCIe) and their size-table neighbourhood
-  const int64_t per_cta = (total + gridDim.x - 1) / gridDim.x;
-  const int64_t first = (int64_t)blockIdx.x * per_cta, step = 1;
-  const int64_t n_mine = first < total ? (total - first < per_cta ? total - first : per_cta) : 0;
+  const int64_t per_pipe = (total + vgrid - 1) / vgrid;
+  const int64_t first = vcta * per_pipe, step = 1;
+  const int64_t n_mine = first < total ? (total - first < per_pipe ? total - first : per_pipe) : 0;
   // thread 0 keeps the ids of the pair it is working on and asks for the next pair's early
   int32_t id_pair = -1;
   int64_t id_g = 0, id_c = 0, nx_g = 0, nx_c = 0;
@@ -159,17 +181,15 @@ __global__ void __launch_bounds__(kThreads, 2) kv_quant_fp8_kernel(const __grid_
       if (it + kInStages - 1 < n_mine) issue_load(it + kInStages - 1);
       if (it >= 2) ptx::bulk_wait_read<1>();   // the store of tile it-2 has finished reading out[ob]
     }
-    __syncthreads();
-    int ok = ptx::mbar_wait_bounded(&full[st], (phases >> st) & 1u, kWaitBudgetNs) ? 1 : 0;
+    pipe_sync<T>(pipe);
+    if (!ptx::mbar_wait_bounded(&full[st], (phases >> st) & 1u, kWaitBudgetNs)) s_abort = 1;
     phases ^= 1u << st;
-    if (!__syncthreads_and(ok)) {
-      if (tid == 0) s_abort = 1;
-      break;
-    }
+    pipe_sync<T>(pipe);
+    if (*reinterpret_cast<volatile int*>(&s_abort)) break;      // the pipeline leaves together
     const int elems = s_elems[st];
     const int groups = elems / kQuantGroup;      // a multiple of 4: a warp's four groups are there or not together
     const int l8 = lane % kLanesPerGroup;        // this lane's values: 8 * l8 .. + 7 of either half of its group
-    for (int gidx = warp * 4 + lane / kLanesPerGroup; gidx < groups; gidx += kThreads / kLanesPerGroup) {
+    for (int gidx = warp * 4 + lane / kLanesPerGroup; gidx < groups; gidx += T / kLanesPerGroup) {
       if (PACK) {
         const uint4* src = reinterpret_cast<const uint4*>(sm.in[st]) + gidx * (kQuantGroup / 8) + l8;
         const uint4 a = src[0], b = src[kLanesPerGroup];
@@ -198,7 +218,7 @@ __global__ void __launch_bounds__(kThreads, 2) kv_quant_fp8_kernel(const __grid_
       }
     }
     ptx::fence_proxy_async_smem();   // generic-proxy writes to out[] before the bulk store reads them
-    __syncthreads();
+    pipe_sync<T>(pipe);
     if (tid == 0) {
       if (elems > 0) {
         if (PACK) {
@@ -220,30 +240,49 @@ __global__ void __launch_bounds__(kThreads, 2) kv_quant_fp8_kernel(const __grid_
   }
 }
 
+template <bool PACK, int T>
+constexpr int pipe_smem() { return (int)sizeof(Smem<PACK, T>) * Pipe<T>::kGroups; }
+
+template <bool PACK, int T>
+cudaError_t load_pipe() {
+  return cudaFuncSetAttribute(kv_quant_fp8_kernel<PACK, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              pipe_smem<PACK, T>());
+}
+
+template <bool PACK, int T>
+cudaError_t launch_pipe(const KvCopyParams& p, int num_ctas, cudaStream_t stream) {
+  const cudaError_t e = load_pipe<PACK, T>();
+  if (e != cudaSuccess) return e;
+  const int tiles_per_chunk = (int)((p.chunk_bytes / 2 + Pipe<T>::kTileElems - 1) / Pipe<T>::kTileElems);
+  const int64_t total = (int64_t)p.num_pairs * p.num_layers * p.kv_dim * tiles_per_chunk;
+  const int64_t need = (total + Pipe<T>::kGroups - 1) / Pipe<T>::kGroups;
+  const int64_t ctas = num_ctas > 0 ? num_ctas : 32;
+  kv_quant_fp8_kernel<PACK, T><<<(unsigned)(ctas < need ? ctas : need), kCtaThreads, pipe_smem<PACK, T>(), stream>>>(
+      p, tiles_per_chunk);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t kv_quant_load_kernels() {
-  const cudaError_t e = cudaFuncSetAttribute(kv_quant_fp8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(Smem<false>));
-  return e != cudaSuccess ? e : cudaFuncSetAttribute(kv_quant_fp8_kernel<true>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<true>));
+  cudaError_t e = load_pipe<false, 256>();
+  if (e == cudaSuccess) e = load_pipe<true, 256>();
+  if (e == cudaSuccess) e = load_pipe<false, 128>();
+  if (e == cudaSuccess) e = load_pipe<true, 128>();
+  if (e == cudaSuccess) e = load_pipe<false, 64>();
+  if (e == cudaSuccess) e = load_pipe<true, 64>();
+  return e;
 }
 
 cudaError_t launch_kv_quant_fp8(const KvCopyParams& p, int num_ctas, cudaStream_t stream) {
   if (p.num_pairs <= 0 || p.num_layers <= 0 || p.kv_dim <= 0 || p.chunk_bytes <= 0) return cudaSuccess;
   const int64_t chunk_elems = p.chunk_bytes / 2;
   if ((p.chunk_bytes & 1) || chunk_elems % 512 != 0 || !kv_copy_tma_eligible(p)) return cudaErrorInvalidValue;
-  const int tiles_per_chunk = (int)((chunk_elems + kTileElems - 1) / kTileElems);
-  const int64_t total = (int64_t)p.num_pairs * p.num_layers * p.kv_dim * tiles_per_chunk;
-  int ctas = num_ctas > 0 ? num_ctas : 32;
-  if ((int64_t)ctas > total) ctas = (int)total;
-  const cudaError_t e = kv_quant_load_kernels();
-  if (e != cudaSuccess) return e;
-  if (p.h2d)
-    kv_quant_fp8_kernel<false><<<ctas, kThreads, sizeof(Smem<false>), stream>>>(p, tiles_per_chunk);
-  else
-    kv_quant_fp8_kernel<true><<<ctas, kThreads, sizeof(Smem<true>), stream>>>(p, tiles_per_chunk);
-  return cudaGetLastError();
+  if (chunk_elems <= Pipe<64>::kTileElems)
+    return p.h2d ? launch_pipe<false, 64>(p, num_ctas, stream) : launch_pipe<true, 64>(p, num_ctas, stream);
+  if (chunk_elems <= Pipe<128>::kTileElems)
+    return p.h2d ? launch_pipe<false, 128>(p, num_ctas, stream) : launch_pipe<true, 128>(p, num_ctas, stream);
+  return p.h2d ? launch_pipe<false, 256>(p, num_ctas, stream) : launch_pipe<true, 256>(p, num_ctas, stream);
 }
 
 }  // namespace fkv

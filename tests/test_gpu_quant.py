@@ -66,6 +66,47 @@ def test_pack_unpack_match_reference(shape):
             assert bool((err <= bound).all())
 
 
+@pytest.mark.parametrize("elems", [512, 1536, 2048, 2560, 4096, 4608])       # 64, 128 and 256 threads per tile
+@pytest.mark.parametrize("ctas", [3, 48])
+def test_small_chunks_pack_to_the_reference_bytes_and_back(elems, ctas):
+    dev = torch.device("cuda:0")
+    shape = KVShape("s", 3, 1, elems // 8, tokens_per_block=8)
+    NB, n = 90, 71
+    kv, layout = alloc_paged_cache(shape, NB, dev, "vllm", fill="normal", seed=64)
+    # scales over the whole range of bf16, so that quotients meet rounding boundaries, zeros and saturation
+    kv[0].mul_(torch.exp(12 * torch.randn(kv[0].shape[:-1], device=dev)).unsqueeze(-1).to(torch.bfloat16))
+    kv[1][0].copy_((torch.randint(-64, 65, kv[1][0].shape, device=dev) * 7).to(torch.bfloat16))      # exact halves
+    kv[2][1].zero_()
+    reg = register_tensors(kv, layout)
+    E = reg.chunk_bytes // 2
+    assert E == elems
+    pc = packed_chunk_bytes(E)
+    L, K = shape.num_layers, shape.kv_dim
+    pool = torch.zeros(NB, L, K, pc, dtype=torch.uint8).pin_memory()
+    host = HostSide(pool.data_ptr(), K * pc, pc, L * K * pc, NB)
+    rng = np.random.default_rng(4)
+    g, c, g2 = (rng.permutation(NB)[:n].astype(np.int64) for _ in range(3))
+    status = new_status(dev)
+    keep = kv_quant_fp8(reg, host, g, c, h2d=False, num_ctas=ctas, status=status)
+    torch.cuda.synchronize()
+    gi, gi2, ci = torch.from_numpy(g).to(dev), torch.from_numpy(g2).to(dev), torch.from_numpy(c)
+    want = {}
+    for l in range(L):
+        for k in range(K):
+            q, s = want[l, k] = reference_pack(kv[l][k][gi].reshape(n, E))
+            got = pool[ci, l, k]
+            assert torch.equal(got[:, :E], q.cpu()), (l, k)
+            assert torch.equal(got[:, E:].contiguous().view(torch.float32), s.cpu()), (l, k)
+    for t in kv:
+        t.zero_()
+    keep += kv_quant_fp8(reg, host, g2, c, h2d=True, num_ctas=ctas, status=status)
+    torch.cuda.synchronize()
+    assert decode_status(status) == 0
+    for l in range(L):
+        for k in range(K):
+            assert torch.equal(kv[l][k][gi2].reshape(n, E).view(torch.int16), reference_unpack(*want[l, k]).view(torch.int16))
+
+
 @pytest.mark.parametrize("shape", [KVShape("l1", 16, 8, 128, tokens_per_block=16),
                                    KVShape("l2", 15, 1, 576, use_mla=True, tokens_per_block=64)])   # ragged last tile
 def test_copy_engine_route_moves_the_same_bytes(shape):
