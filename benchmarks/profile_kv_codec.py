@@ -6,6 +6,7 @@ round trip (bit-exact for the lossless codec). Sized for an ``ncu`` capture of a
 launches: 512 MiB per direction, about 1.5 GiB on the device.
 """
 import argparse
+import dataclasses
 import os
 import sys
 
@@ -28,9 +29,10 @@ def main() -> None:
     ap.add_argument("--iters", type=int, default=2)
     ap.add_argument("--ctas-d2h", type=int, default=48)
     ap.add_argument("--ctas-h2d", type=int, default=32)
+    ap.add_argument("--kv-heads", type=int, default=8, help="KV heads of a page (1: what a rank of 8 holds)")
     a = ap.parse_args()
     dev = torch.device("cuda:0")
-    shape = get_shape("llama3-8b")
+    shape = dataclasses.replace(get_shape("llama3-8b"), num_kv_heads=a.kv_heads)
     kv, layout = alloc_paged_cache(shape, a.pool_blocks, dev, "vllm", fill="normal", seed=1)
     reg = register_tensors(kv, layout)
     elems = reg.chunk_bytes // 2

@@ -137,16 +137,17 @@ void init_kernel_bindings(py::module_& m) {
         throw_on(e, "kv_quant_fp8");
       }, py::arg("params"), py::arg("num_ctas"), py::arg("stream"))
       .def("compress_bf16", [](CodecLink& l, py::dict params, uint64_t size_table_ptr, int layers_total, int num_ctas,
-                               uint64_t stream) {
+                               int staged_ctas, uint64_t stream) {
         KvCopyParams p = kv_params_from_dict(params);
         cudaError_t e;
         {
           py::gil_scoped_release rel;
           e = l.compress_bf16(p, (uint32_t*)(uintptr_t)size_table_ptr, layers_total, num_ctas,
-                              (cudaStream_t)(uintptr_t)stream);
+                              staged_ctas, (cudaStream_t)(uintptr_t)stream);
         }
         throw_on(e, "kv_compress_bf16");
-      }, py::arg("params"), py::arg("size_table_ptr"), py::arg("layers_total"), py::arg("num_ctas"), py::arg("stream"))
+      }, py::arg("params"), py::arg("size_table_ptr"), py::arg("layers_total"), py::arg("num_ctas"),
+         py::arg("staged_ctas"), py::arg("stream"))
       .def_property_readonly("staged_ops", &CodecLink::staged_ops);
   m.def("fp8_packed_chunk_bytes", &fp8_packed_chunk_bytes);
 

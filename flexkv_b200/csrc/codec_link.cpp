@@ -116,7 +116,7 @@ bool plan_rows(const KvCopyParams& p, const uint32_t* sizes, const CeHostRun& pi
 }  // namespace
 
 cudaError_t CodecLink::compress_bf16(const KvCopyParams& p, uint32_t* size_table, int layers_total, int num_ctas,
-                                     cudaStream_t stream) {
+                                     int staged_ctas, cudaStream_t stream) {
   CeStagePlan pl;
   // rows of chunks below 4096 values are too short for a copy engine: 48.2 GB/s at 2048 values, the kernel 50.4
   if (!p.h2d || size_table == nullptr || p.chunk_bytes < 8192 || p.chunk_bytes % 2048 != 0 || layers_total != num_layers_ ||
@@ -140,10 +140,9 @@ cudaError_t CodecLink::compress_bf16(const KvCopyParams& p, uint32_t* size_table
   return ce_copy_staged(
       p, pl, staging_,
       [&](const KvCopyParams& q, int64_t host_block, cudaStream_t s) {
-        // out of the staging buffer: twice the pipelines for a quarter of the time, so that the last piece is short
         const bool staged = q.cpu_base != p.cpu_base;
         return launch_kv_compress_bf16(q, size_table + host_block * row_entries, layers_total,
-                                       staged ? 2 * num_ctas : num_ctas, s);
+                                       staged ? staged_ctas : num_ctas, s);
       },
       stream, &link);
 }

@@ -32,8 +32,9 @@ class CodecLink {
   // staged: only the used bytes of the tile slots cross, as rows of a 2-D copy, each class of tiles (K or V, tile of
   // the chunk) as wide as its largest tile in the piece. Offloads stay with the kernel: the sizes are not known before
   // a piece is packed, and rows of 11 KiB go out at 51.7 GB/s where the kernel reaches 52.5.
+  // `staged_ctas` takes the place of `num_ctas` where the kernel unpacks out of the staging buffer.
   cudaError_t compress_bf16(const KvCopyParams& p, uint32_t* size_table, int layers_total, int num_ctas,
-                            cudaStream_t stream);
+                            int staged_ctas, cudaStream_t stream);
   uint64_t staged_ops() const { return staged_ops_; }
 
  private:

@@ -335,16 +335,19 @@ OpResult TransferGroup::transfer(const int64_t* gpu_blocks, const int64_t* cpu_b
   Rank& rk = *ranks_[0];
   int before = -1;
   if (cudaGetDevice(&before) != cudaSuccess) before = -1;
-  {
+  int status = -(int)cudaErrorUnknown;
+  float ms = 0.f;
+  try {
     // behind what the rank's thread has in hand; it takes nothing new meanwhile
     std::lock_guard<std::mutex> exec(rk.exec_mu);
-    float ms = 0.f;
-    cudaError_t e = before == gpus_[0].device ? cudaSuccess : cudaSetDevice(gpus_[0].device);
-    int status;
-    if (e == cudaSuccess) status = retire_task(0, launch_task(0, t, 0), 0, ms);
-    else status = -(int)e;
-    finish(t.ticket, status, ms);
+    const cudaError_t e = before == gpus_[0].device ? cudaSuccess : cudaSetDevice(gpus_[0].device);
+    status = e == cudaSuccess ? retire_task(0, launch_task(0, t, 0), 0, ms) : -(int)e;
+  } catch (...) {
+    finish(t.ticket, status, 0.f);      // gives the id ring slot back
+    wait(t.ticket);
+    throw;
   }
+  finish(t.ticket, status, ms);
   if (before >= 0 && before != gpus_[0].device) cudaSetDevice(before);
   return wait(t.ticket);
 }

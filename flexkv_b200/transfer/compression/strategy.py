@@ -12,13 +12,15 @@ from __future__ import annotations
 from typing import Any, Dict
 
 from ... import _native
+from ...storage.storage_engine import host_register_chunk_bytes
 
 
 def codec_link(worker: Any, staging_bytes: int):
     """The native router of a worker's ops between kernel and copy engines, or None where every op belongs to the
-    kernel: an engine of the user's choice (FLEXKV_TRANSFER_ENGINE), or several ranks behind one op, whose slices of a
-    host block are not one span and whose launches read the same id arrays."""
-    if len(worker.regs) != 1 or not worker.copy_engines:
+    kernel: an engine of the user's choice (FLEXKV_TRANSFER_ENGINE), several ranks behind one op, whose slices of a
+    host block are not one span and whose launches read the same id arrays, or a host pool registered in parts, which
+    a driver copy must not straddle."""
+    if len(worker.regs) != 1 or not worker.copy_engines or host_register_chunk_bytes():
         return None
     reg = worker.regs[0]
     return _native.C.CodecLink(reg.device_id, reg.num_layers, reg.kv_dim, worker.kv_stride, staging_bytes)
@@ -87,9 +89,8 @@ class Fp8BlockScaleStrategy(CompressionStrategy):
 
 
 class ExponentPackStrategy(CompressionStrategy):
-    """Lossless bf16 codec: sign+mantissa bytes stay raw, every group of 128 values stores its
-    largest exponent once and each value's distance to it in w bits, w chosen per group
-    (about 0.75x bytes on unit-normal data)."""
+    """Lossless bf16 codec: sign+mantissa bytes stay raw, exponents are prefix coded by their frequency
+    rank in the tile (about 0.68x bytes on unit-normal data)."""
     name = "bf16_xp"
     TILE_ELEMS = 8192
     TILE_SLOT = 2 * TILE_ELEMS + 128
@@ -123,7 +124,7 @@ class ExponentPackStrategy(CompressionStrategy):
         off = self.spec.rank_offset_entries(rank_index)
         table, layers = self.size_table.data_ptr() + 4 * off, self.spec.kernel_layers()
         if self._link is not None:
-            self._link.compress_bf16(params, table, layers, num_ctas, stream)
+            self._link.compress_bf16(params, table, layers, num_ctas, self.worker.staged_num_ctas, stream)
         else:
             _native.C.kv_compress_bf16(params, table, layers, num_ctas, stream)
 

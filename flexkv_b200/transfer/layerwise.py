@@ -26,6 +26,7 @@ from .. import _native
 from ..common.config import GLOBAL_CONFIG_FROM_ENV
 from ..common.debug import flexkv_logger
 from ..common.transfer import LayerwiseTransferOp, TransferOp, WorkerKey
+from ..storage.storage_engine import host_register_chunk_bytes
 from .workers import OpOutcome, TransferWorker, _launch_cfg
 
 HEADER = struct.Struct("iiii")
@@ -164,8 +165,11 @@ def build_layerwise_group(storage, model_config, key: WorkerKey, notify_mode: Op
         layer_stride, kv_stride, tp_stride = host.layer_stride, host.kv_stride, host.chunk_bytes // n_slices
     host_d = dict(base=host.base, layer_stride=layer_stride, kv_stride=kv_stride, block_stride=host.block_bytes,
                   num_blocks=host.num_blocks)
+    h2d = _launch_cfg(env, True)
+    if host_register_chunk_bytes() and h2d["engine"] >= 2:
+        h2d["engine"] = 0           # a host pool registered in parts: driver copies must not straddle two of them
     opts = dict(num_layers=reg0.num_layers, kv_dim=reg0.kv_dim, chunk_bytes=reg0.chunk_bytes,
-                cpu_tp_stride=tp_stride, shared_kv=shared, h2d=_launch_cfg(env, True), d2h=_launch_cfg(env, False),
+                cpu_tp_stride=tp_stride, shared_kv=shared, h2d=h2d, d2h=_launch_cfg(env, False),
                 max_blocks_per_op=max(4096, min(1 << 18, host.num_blocks)),
                 notify_mode=notify_mode or env.layerwise_notify_mode, num_counters=num_counters,
                 layers_per_batch=layers_per_batch, create_eventfds=create_eventfds)

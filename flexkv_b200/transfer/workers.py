@@ -374,6 +374,9 @@ class QuantGpuHostWorker(TransferWorker):
         # traffic; the fp8 kernel needs fewer (its CTAs are single pipelines)
         dflt = 80 if storage.host.quant == "bf16_xp" else (32 if h2d else 48)
         self.num_ctas = int(os.environ.get("FLEXKV_QUANT_NUM_CTA", dflt))
+        # unpacking out of the staging buffer: twice the pipelines for a quarter of the time, so that the restore's
+        # last piece is short; a user's own figure stands
+        self.staged_num_ctas = self.num_ctas if "FLEXKV_QUANT_NUM_CTA" in os.environ else 2 * dflt
         self._torch = torch
         self.streams = {r.device_id: torch.cuda.Stream(device=r.device_id) for r in self.regs}
         # Kept between ops, which this worker runs one at a time: pinned id buffers and status words that the kernels

@@ -62,3 +62,13 @@ def test_strategy_geometry():
     x = strategy_for("bf16_xp")
     assert isinstance(x, ExponentPackStrategy) and x.lossless and x.needs_size_table
     assert x.host_chunk_bytes(16384, 2) == 2 * (2 * 8192 + 128)
+
+
+def test_ops_that_belong_to_the_kernel_get_no_copy_engine_link(monkeypatch):
+    from types import SimpleNamespace as N
+
+    from flexkv_b200.transfer.compression.strategy import codec_link
+    assert codec_link(N(regs=[1, 2], copy_engines=True), 1 << 20) is None      # several ranks read one id array
+    assert codec_link(N(regs=[1], copy_engines=False), 1 << 20) is None        # an engine of the user's choice
+    monkeypatch.setenv("FLEXKV_HOST_REGISTER_CHUNK_BYTES", str(1 << 30))
+    assert codec_link(N(regs=[1], copy_engines=True), 1 << 20) is None         # copies must not straddle registrations

@@ -185,7 +185,7 @@ def test_restore_through_the_copy_engines_matches_the_kernel(shape, spread):
     g2 = rng.permutation(NB)[:c.size].astype(np.int64)
     ids = [torch.from_numpy(a.copy()).pin_memory() for a in (g2, c)]
     link = _native.C.CodecLink(0, L, K, slot, 8 << 20)
-    link.compress_bf16(make_params(reg, host, *ids, True, status_ptr=status.data_ptr()), table.data_ptr(), L, 80,
+    link.compress_bf16(make_params(reg, host, *ids, True, status_ptr=status.data_ptr()), table.data_ptr(), L, 80, 160,
                        torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     assert decode_status(status) == 0 and link.staged_ops == 1
@@ -198,7 +198,7 @@ def test_restore_through_the_copy_engines_matches_the_kernel(shape, spread):
         assert not bool(t[:, other.to(dev)].view(torch.int16).any())
     # a slot that was never written: every size that is there is restored, the error is reported
     table.view(NB, -1)[c[10], 3] = 0
-    link.compress_bf16(make_params(reg, host, *ids, True, status_ptr=status.data_ptr()), table.data_ptr(), L, 80,
+    link.compress_bf16(make_params(reg, host, *ids, True, status_ptr=status.data_ptr()), table.data_ptr(), L, 80, 160,
                        torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     assert decode_status(status) == 16
