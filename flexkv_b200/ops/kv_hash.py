@@ -14,10 +14,14 @@ from ..common.block import namespace_prefix
 
 def gpu_block_hashes(seqs: Sequence[torch.Tensor], tokens_per_block: int, namespace: Optional[List[str]] = None,
                      stream: Optional[torch.cuda.Stream] = None) -> List[torch.Tensor]:
-    """``seqs``: int64 CUDA tensors (one per sequence, same device). Returns one uint64-valued
+    """``seqs``: int64 CUDA tensors (one per sequence, same device; ``ValueError`` otherwise). Returns one uint64-valued
     int64 CUDA tensor of block keys per sequence (view with ``.view(torch.uint64)`` or copy to numpy)."""
     if not seqs:
         return []
+    # the kernel reads these addresses: memory of the host or of another GPU must not get there
+    where = [t.get_device() for t in seqs]
+    if where.count(where[0]) != len(where) or not seqs[0].is_cuda:
+        raise ValueError("gpu_block_hashes: every sequence must be a CUDA tensor on the device of the first")
     dev = seqs[0].device
     C = _native.C
     s = stream if stream is not None else torch.cuda.current_stream(dev)
@@ -30,7 +34,8 @@ def gpu_block_hashes(seqs: Sequence[torch.Tensor], tokens_per_block: int, namesp
         s.wait_stream(torch.cuda.current_stream(dev))
     if len(seqs) <= C.HASH_LIST_SEQS and (ns is None or ns.size <= C.HASH_LIST_NS) and max(lens) < 2**31:
         # the sequences stay where they are: addresses, lengths and prefix travel in the launch parameters
-        seqs = [t if t.dtype == torch.int64 and t.is_contiguous() else t.to(torch.int64).contiguous() for t in seqs]
+        i64 = torch.int64
+        seqs = [t if t.dtype is i64 and t.is_contiguous() else t.to(i64).contiguous() for t in seqs]
         C.kv_block_hashes_list([t.data_ptr() for t in seqs], lens, int(tokens_per_block),
                                b"" if ns is None else ns.astype(np.uint8).tobytes(), out.data_ptr(), s.cuda_stream)
         if side:

@@ -49,3 +49,12 @@ def test_segment_edges_and_both_forms(nseq, lens, tpb, namespace):
     torch.cuda.synchronize()
     for i in sorted({0, 1, 2, nseq // 2, nseq - 2, nseq - 1}):
         assert got[i].cpu().numpy().view(np.uint64).tolist() == hash_blocks(seqs[i], tpb, namespace).tolist()
+
+
+@pytest.mark.parametrize("count", [2, 200])
+def test_host_tensor_among_the_sequences_is_refused(count):
+    dev = torch.device("cuda:0")
+    seqs = [torch.arange(64, device=dev) for _ in range(count)]
+    seqs[-1] = torch.arange(64)
+    with pytest.raises(ValueError):
+        gpu_block_hashes(seqs, 16)
