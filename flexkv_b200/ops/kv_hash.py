@@ -29,13 +29,14 @@ def gpu_block_hashes(seqs: Sequence[torch.Tensor], tokens_per_block: int, namesp
     nblk = [n // tokens_per_block for n in lens]
     ns = namespace_prefix(namespace)
     out = torch.empty(sum(nblk), dtype=torch.int64, device=dev)
-    side = s != torch.cuda.current_stream(dev)
-    if side:
-        s.wait_stream(torch.cuda.current_stream(dev))
+    current = torch.cuda.current_stream(dev)
+    side = s != current
     if len(seqs) <= C.HASH_LIST_SEQS and (ns is None or ns.size <= C.HASH_LIST_NS) and max(lens) < 2**31:
         # the sequences stay where they are: addresses, lengths and prefix travel in the launch parameters
         i64 = torch.int64
         seqs = [t if t.dtype is i64 and t.is_contiguous() else t.to(i64).contiguous() for t in seqs]
+        if side:
+            s.wait_stream(current)          # behind the conversions
         C.kv_block_hashes_list([t.data_ptr() for t in seqs], lens, int(tokens_per_block),
                                b"" if ns is None else ns.astype(np.uint8).tobytes(), out.data_ptr(), s.cuda_stream)
         if side:
@@ -46,6 +47,8 @@ def gpu_block_hashes(seqs: Sequence[torch.Tensor], tokens_per_block: int, namesp
     offs = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int64, device=dev)
     ooffs = torch.tensor(np.concatenate([[0], np.cumsum(nblk)]), dtype=torch.int64, device=dev)
     ns_t = torch.from_numpy(np.ascontiguousarray(ns, dtype=np.int64)).to(dev) if ns is not None and len(ns) else None
+    if side:
+        s.wait_stream(current)              # behind the concatenation and the uploads
     C.kv_block_hashes(flat.data_ptr(), offs.data_ptr(), len(seqs), int(tokens_per_block),
                       ns_t.data_ptr() if ns_t is not None else 0, int(ns_t.numel()) if ns_t is not None else 0,
                       out.data_ptr(), ooffs.data_ptr(), s.cuda_stream)

@@ -92,3 +92,16 @@ def test_sequences_elsewhere_are_refused_before_any_launch(rig, stranger, count)
     with pytest.raises(ValueError):
         kv_hash.gpu_block_hashes(_seqs(1, OnHost), 16, stream=rig.side)
     assert not [e for e in rig.log if e[0] == "launch"]
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+@pytest.mark.parametrize("count", [3, 200])
+def test_a_side_stream_waits_for_the_conversions(rig, count, dtype):
+    """Conversions, concatenations and uploads run on the current stream; the other stream is told to wait for it after
+    the last of them and before the launch."""
+    seqs = _seqs(count, dtype=dtype)
+    seqs[1] = seqs[1][::2]
+    kv_hash.gpu_block_hashes(seqs, 16, stream=rig.side)
+    what = [e[0] for e in rig.log]
+    last = max(i for i, w in enumerate(what) if w == "convert")
+    assert last < what.index("wait") < what.index("launch") and what.count("wait") == 1

@@ -58,3 +58,18 @@ def test_host_tensor_among_the_sequences_is_refused(count):
     seqs[-1] = torch.arange(64)
     with pytest.raises(ValueError):
         gpu_block_hashes(seqs, 16)
+
+
+@pytest.mark.parametrize("count", [5, 130])
+def test_side_stream_reads_converted_inputs(count):
+    dev = torch.device("cuda:0")
+    rng = np.random.default_rng(count)
+    full = [rng.integers(0, 128256, size=4096 + i, dtype=np.int64) for i in range(count)]
+    seqs = [torch.from_numpy(f).to(dev) for f in full]
+    seqs = [t.to(torch.int32) if i % 2 else t[::2] for i, t in enumerate(seqs)]
+    side = torch.cuda.Stream(dev)
+    torch.cuda._sleep(2_000_000)            # a millisecond of work in front of the conversions
+    got = gpu_block_hashes(seqs, 16, stream=side)
+    side.synchronize()
+    for i, (f, g) in enumerate(zip(full, got)):
+        assert g.cpu().numpy().view(np.uint64).tolist() == hash_blocks(f if i % 2 else f[::2].copy(), 16).tolist()
