@@ -15,7 +15,11 @@ from ..common.block import namespace_prefix
 def gpu_block_hashes(seqs: Sequence[torch.Tensor], tokens_per_block: int, namespace: Optional[List[str]] = None,
                      stream: Optional[torch.cuda.Stream] = None) -> List[torch.Tensor]:
     """``seqs``: int64 CUDA tensors (one per sequence, same device; ``ValueError`` otherwise). Returns one uint64-valued
-    int64 CUDA tensor of block keys per sequence (view with ``.view(torch.uint64)`` or copy to numpy)."""
+    int64 CUDA tensor of block keys per sequence (view with ``.view(torch.uint64)`` or copy to numpy).
+
+    With a ``stream`` of its own the keys are computed there, behind what the current stream holds. Several sequences
+    are copied first, in the order of the current stream, which may then overwrite them; a single one is read where it
+    is and has to stay until ``stream`` has passed the call."""
     if not seqs:
         return []
     # the kernel reads these addresses: memory of the host or of another GPU must not get there
@@ -32,11 +36,15 @@ def gpu_block_hashes(seqs: Sequence[torch.Tensor], tokens_per_block: int, namesp
     current = torch.cuda.current_stream(dev)
     side = s != current
     if len(seqs) <= C.HASH_LIST_SEQS and (ns is None or ns.size <= C.HASH_LIST_NS) and max(lens) < 2**31:
-        # the sequences stay where they are: addresses, lengths and prefix travel in the launch parameters
+        # addresses, lengths and prefix travel in the launch parameters; on the current stream the sequences are read
+        # where they are
         i64 = torch.int64
-        seqs = [t if t.dtype is i64 and t.is_contiguous() else t.to(i64).contiguous() for t in seqs]
+        if side and len(seqs) > 1:
+            seqs = list(torch.cat([t.reshape(-1).to(i64) for t in seqs]).split(lens))
+        else:
+            seqs = [t if t.dtype is i64 and t.is_contiguous() else t.to(i64).contiguous() for t in seqs]
         if side:
-            s.wait_stream(current)          # behind the conversions
+            s.wait_stream(current)          # behind the copies
         C.kv_block_hashes_list([t.data_ptr() for t in seqs], lens, int(tokens_per_block),
                                b"" if ns is None else ns.astype(np.uint8).tobytes(), out.data_ptr(), s.cuda_stream)
         if side:

@@ -105,3 +105,21 @@ def test_a_side_stream_waits_for_the_conversions(rig, count, dtype):
     what = [e[0] for e in rig.log]
     last = max(i for i, w in enumerate(what) if w == "convert")
     assert last < what.index("wait") < what.index("launch") and what.count("wait") == 1
+
+
+@pytest.mark.parametrize("count,in_place", [(1, True), (3, False), (200, False)])
+def test_a_side_stream_reads_copies(rig, count, in_place):
+    """Several sequences are copied in the order of the current stream, so that the caller may go on to overwrite them
+    there while the keys are computed on the other stream."""
+    seqs = _seqs(count)
+    mine = {t.data_ptr() for t in seqs}
+    kv_hash.gpu_block_hashes(seqs, 16, stream=rig.side)
+    read = [e[1] for e in rig.log if e[0] == "launch"][0]
+    assert all((p in mine) == in_place for p in read)
+    assert set(read) <= {e[1] for e in rig.log if e[0] == "keep"}
+
+
+def test_the_current_stream_reads_in_place(rig):
+    seqs = _seqs(4)
+    kv_hash.gpu_block_hashes(seqs, 16)
+    assert rig.log == [("launch", [t.data_ptr() for t in seqs])]
