@@ -220,6 +220,10 @@ void init_kernel_bindings(py::module_& m) {
              "kv_block_hashes launch");
   }, py::arg("tokens"), py::arg("lens"), py::arg("tokens_per_block"), py::arg("ns") = py::bytes(), py::arg("out") = 0,
      py::arg("stream") = 0);
+  m.def("hash_extent", [](int64_t ntok, int64_t ns_len, int64_t tokens_per_block) {
+    const HashExtent x = hash_extent(ntok, ns_len, tokens_per_block);
+    return py::make_tuple(x.blocks, x.stripes);
+  }, py::arg("ntok"), py::arg("ns_len"), py::arg("tokens_per_block"));
   m.attr("HASH_LIST_SEQS") = kHashListSeqs;
   m.attr("HASH_LIST_NS") = kHashListNs;
 

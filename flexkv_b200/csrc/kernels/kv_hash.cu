@@ -42,10 +42,11 @@ struct HashParams {
   const int64_t* ns;                  // prefix values in memory; null = ns8
   uint64_t* out;
   int64_t num_seqs;
-  int32_t tpb, ns_len;
+  int64_t ns_len;
+  int32_t tpb;
   const int64_t* list_tokens[kHashListSeqs];
   int32_t list_len[kHashListSeqs];
-  uint32_t list_out[kHashListSeqs];   // first key of the sequence in `out`
+  uint64_t list_out[kHashListSeqs];   // first key of the sequence in `out`
   uint8_t ns8[kHashListNs];
 };
 
@@ -58,8 +59,8 @@ __global__ void __launch_bounds__(kHashThreads) kv_block_hashes_kernel(const __g
   __shared__ uint64_t s_acc[2][G * SEGW];              // the four accumulators after each stripe
   __shared__ const int64_t* s_tok[G];
   __shared__ uint64_t* s_out[G];
-  __shared__ int32_t s_stripes[G], s_blocks[G];
-  __shared__ int s_segs;
+  __shared__ int64_t s_stripes[G], s_blocks[G];
+  __shared__ unsigned long long s_segs;
   const int tid = threadIdx.x;
   if (tid == 0) s_segs = 0;
   __syncthreads();
@@ -80,14 +81,13 @@ __global__ void __launch_bounds__(kHashThreads) kv_block_hashes_kernel(const __g
         s_out[tid] = p.out + p.list_out[seq];
       }
     }
-    const int32_t nblk = (int32_t)(ntok / p.tpb);
-    const int32_t stripes = nblk > 0 ? (int32_t)(((int64_t)p.ns_len + (int64_t)nblk * p.tpb) >> 2) : 0;
-    s_blocks[tid] = nblk;
-    s_stripes[tid] = stripes;
-    if (nblk > 0) atomicMax(&s_segs, max(1, (stripes + SEG - 1) / SEG));
+    const HashExtent x = hash_extent(ntok, p.ns_len, p.tpb);
+    s_blocks[tid] = x.blocks;
+    s_stripes[tid] = x.stripes;
+    if (x.blocks > 0) atomicMax(&s_segs, (unsigned long long)max((int64_t)1, (x.stripes + SEG - 1) / SEG));
   }
   __syncthreads();
-  const int segs = s_segs;
+  const int32_t segs = (int32_t)s_segs;                // of 1024 words or 128: 2^31 of them are beyond any memory
   auto word = [&](int g, int64_t i) -> uint64_t {      // i-th word of the stream of sequence g
     if (i >= p.ns_len) return (uint64_t)__ldg(s_tok[g] + (i - p.ns_len));
     return p.ns ? (uint64_t)p.ns[i] : (uint64_t)p.ns8[i];
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kHashThreads) kv_block_hashes_kernel(const __g
     for (int i = t; i < G * SEGW; i += threads) {
       const int g = i / SEGW;
       const int64_t w = (int64_t)seg * SEGW + i % SEGW;
-      if (w < (int64_t)s_stripes[g] * 4) s_in[seg & 1][i] = word(g, w) * P2;
+      if (w < s_stripes[g] * 4) s_in[seg & 1][i] = word(g, w) * P2;
     }
   };
   // number of blocks whose digest covers at most `stripes` complete stripes
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kHashThreads) kv_block_hashes_kernel(const __g
   };
   auto digest = [&](int seg, int t, int threads) {
     for (int g = 0; g < G; ++g) {
-      const int64_t hi = min((int64_t)s_blocks[g], blocks_upto((int64_t)(seg + 1) * SEG));
+      const int64_t hi = min(s_blocks[g], blocks_upto((int64_t)(seg + 1) * SEG));
       for (int64_t b = (seg == 0 ? 0 : blocks_upto((int64_t)seg * SEG)) + t; b < hi; b += threads) {
         const int64_t n = p.ns_len + (b + 1) * p.tpb;  // words covered by this digest
         const int64_t stripes = n >> 2;
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kHashThreads) kv_block_hashes_kernel(const __g
       if (seg < segs && cg < G) {
         const uint64_t* in = &s_in[seg & 1][cg * SEGW + q];
         uint64_t* st = &s_acc[seg & 1][cg * SEGW + q];
-        const int cnt = min(SEG, s_stripes[cg] - seg * SEG);
+        const int cnt = (int)min((int64_t)SEG, s_stripes[cg] - (int64_t)seg * SEG);
         int s = 0;
         for (; s + 8 <= cnt; s += 8) {
           uint64_t x[8];
@@ -176,7 +176,7 @@ cudaError_t launch_kv_block_hashes(const int64_t* tokens, const int64_t* offsets
                                    const int64_t* ns_prefix, int64_t ns_len, uint64_t* out, const int64_t* out_offsets,
                                    cudaStream_t stream) {
   if (num_seqs <= 0) return cudaSuccess;
-  if (tokens_per_block <= 0 || ns_len < 0 || ns_len > INT32_MAX || (ns_len > 0 && ns_prefix == nullptr))
+  if (tokens_per_block <= 0 || ns_len < 0 || (ns_len > 0 && ns_prefix == nullptr))
     return cudaErrorInvalidValue;
   HashParams p{};
   p.tokens = tokens;
@@ -186,7 +186,7 @@ cudaError_t launch_kv_block_hashes(const int64_t* tokens, const int64_t* offsets
   p.out = out;
   p.num_seqs = num_seqs;
   p.tpb = tokens_per_block;
-  p.ns_len = (int32_t)ns_len;
+  p.ns_len = ns_len;
   return launch(p, stream);
 }
 
@@ -207,10 +207,9 @@ cudaError_t launch_kv_block_hashes_list(const int64_t* const* tokens, const int6
     if (lens[i] < 0 || lens[i] > INT32_MAX) return cudaErrorInvalidValue;
     p.list_tokens[i] = tokens[i];
     p.list_len[i] = (int32_t)lens[i];
-    p.list_out[i] = (uint32_t)keys;
-    keys += (uint64_t)(lens[i] / tokens_per_block);
+    p.list_out[i] = keys;
+    keys += (uint64_t)hash_extent(lens[i], ns_len, tokens_per_block).blocks;
   }
-  if (keys > UINT32_MAX) return cudaErrorInvalidValue;
   return launch(p, stream);
 }
 

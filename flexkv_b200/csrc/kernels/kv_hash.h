@@ -10,6 +10,16 @@
 
 namespace fkv {
 
+// What a sequence of `ntok` tokens behind a prefix of `ns_len` words comes to: keys, and the complete stripes of four
+// words that its last key covers. 64 bits: with one token per block 2^31 tokens are 16 GiB.
+struct HashExtent {
+  int64_t blocks, stripes;
+};
+__host__ __device__ constexpr HashExtent hash_extent(int64_t ntok, int64_t ns_len, int64_t tokens_per_block) {
+  const int64_t blocks = ntok / tokens_per_block;
+  return {blocks, blocks > 0 ? (ns_len + blocks * tokens_per_block) >> 2 : 0};
+}
+
 // tokens: all sequences back to back; offsets[n+1] (in tokens) and out_offsets[n+1] (in blocks)
 // are device- or mapped-host-readable. ns_prefix (ns_len int64 values, may be null) is fed
 // before every sequence.

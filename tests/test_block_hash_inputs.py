@@ -123,3 +123,11 @@ def test_the_current_stream_reads_in_place(rig):
     seqs = _seqs(4)
     kv_hash.gpu_block_hashes(seqs, 16)
     assert rig.log == [("launch", [t.data_ptr() for t in seqs])]
+
+
+@pytest.mark.parametrize("ntok", [0, 15, 16, 4099, 2**31 - 1, 2**31, 2**33 + 5])
+@pytest.mark.parametrize("tpb,ns_len", [(1, 0), (16, 7), (64, 300)])
+def test_extent_of_a_sequence(ntok, tpb, ns_len):
+    """Keys and stripes of a sequence, as the kernel splits its work: both go beyond 32 bits with short blocks."""
+    blocks = ntok // tpb
+    assert kv_hash._native.C.hash_extent(ntok, ns_len, tpb) == (blocks, (ns_len + blocks * tpb) // 4 if blocks else 0)
