@@ -1,5 +1,7 @@
 #include "kv_quant.h"
 
+#include <cfloat>
+
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
@@ -41,6 +43,12 @@ __device__ __forceinline__ void pipe_sync(int pipe) {
   asm volatile("bar.sync %0, %1;" ::"r"(pipe + 1), "n"(T) : "memory");
 }
 
+// The scale of a group with this largest magnitude. Below FLT_MIN it would be flushed to zero (the build flushes
+// subnormals) and its reciprocal would be infinite: zeros would become NaN codes, all else the largest code.
+__device__ __forceinline__ float group_scale(float amax) {
+  return amax > 0.f ? fmaxf(__fdiv_rn(amax, 448.f), FLT_MIN) : 1.f;
+}
+
 // largest value among the lanes that hold a group
 __device__ __forceinline__ float group_max(float v) {
 #pragma unroll
@@ -56,7 +64,8 @@ __device__ __forceinline__ float2 bf16x2_floats(uint32_t w) {
 // The e4m3 codes of fdiv_rn(x, scale) for a pair of values. `lo` and `hi` are 1 / scale made smaller and larger by
 // 2^-20, far more than the rounding of the reciprocal and of a product: the quotient lies between x * lo and x * hi,
 // rounding to e4m3 is monotone, so where both have the same code the quotient has it too and no division is needed
-// (one pair in some 5000 is divided). Zero, infinite and NaN operands give the same in both forms.
+// (one pair in some 5000 is divided). That needs a finite 1 / scale, which group_scale() sees to; zero, infinite and
+// NaN values and an infinite scale then give the same in both forms.
 __device__ __forceinline__ uint32_t quant2(float2 x, float scale, float lo, float hi) {
   const uint32_t a = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(x.x, lo), __fmul_rn(x.y, lo)), __NV_SATFINITE, __NV_E4M3);
   const uint32_t b = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(x.x, hi), __fmul_rn(x.y, hi)), __NV_SATFINITE, __NV_E4M3);
@@ -200,7 +209,7 @@ __global__ void __launch_bounds__(kCtaThreads, 2) kv_quant_fp8_kernel(const __gr
         for (int i = 0; i < 4; ++i)
           m = fmaxf(m, fmaxf(fmaxf(fabsf(xa[i].x), fabsf(xa[i].y)), fmaxf(fabsf(xb[i].x), fabsf(xb[i].y))));
         const float amax = group_max(m);
-        const float scale = amax > 0.f ? __fdiv_rn(amax, 448.f) : 1.f;
+        const float scale = group_scale(amax);
         const float inv = __frcp_rn(scale), lo = inv * (1.f - 0x1p-20f), hi = inv * (1.f + 0x1p-20f);
         uint2* dst = reinterpret_cast<uint2*>(sm.out[ob]) + gidx * (kQuantGroup / 8) + l8;
         dst[0] = quant8(xa, scale, lo, hi);

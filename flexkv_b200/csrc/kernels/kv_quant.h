@@ -9,8 +9,8 @@
 // Host chunk format (one (layer, kv, block) chunk of E bf16 values):
 //     [ E bytes e4m3 payload ][ E/128 fp32 scales ]          E % 512 == 0
 // so the host chunk stride is E + E/32 bytes. The arithmetic is exact and
-// reproducible: scale = fdiv_rn(amax, 448), q = cvt_rn_satfinite(fdiv_rn(x, scale)),
-// x' = bf16_rn(float(q) * scale); an all-zero group stores scale 1.
+// reproducible: scale = max(fdiv_rn(amax, 448), FLT_MIN), q = cvt_rn_satfinite(fdiv_rn(x, scale)),
+// x' = bf16_rn(float(q) * scale); subnormal values and products count as zero, an all-zero group stores scale 1.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

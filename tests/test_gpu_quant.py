@@ -107,6 +107,41 @@ def test_small_chunks_pack_to_the_reference_bytes_and_back(elems, ctas):
             assert torch.equal(kv[l][k][gi2].reshape(n, E).view(torch.int16), reference_unpack(*want[l, k]).view(torch.int16))
 
 
+@pytest.mark.parametrize("elems", [512, 4096, 8192])                        # 64, 128 and 256 threads per tile
+def test_groups_of_tiny_values(elems):
+    """Groups whose largest value lies where amax / 448 is no normal float any more, on both sides of the line
+    (448 * FLT_MIN = 5.27e-36) and around the smallest normal value, with zeros and values far below it among them."""
+    dev = torch.device("cuda:0")
+    shape = KVShape("t", 1, 1, elems // 8, tokens_per_block=8)
+    amax = torch.tensor([1e-39, 1.1e-38, 1.2e-38, 1e-37, 1.3e-36, 1.4e-36, 5e-36, 5.4e-36, 1e-35, 1e-33])
+    n = NB = len(amax)
+    kv, layout = alloc_paged_cache(shape, NB, dev, "vllm", fill="normal", seed=65)
+    for t in kv[0]:
+        x = t.float().reshape(NB, -1)
+        x = x.clamp(-1, 1) * (torch.rand_like(x) < 0.7) * 10.0 ** -(torch.rand_like(x) < 0.2).float().mul(3)
+        x[:, ::64] = -1
+        t.copy_((x.double() * amax.to(dev).double().unsqueeze(-1)).reshape(t.shape).to(torch.bfloat16))
+    src = [t.reshape(NB, elems).clone() for t in kv[0]]
+    reg = register_tensors(kv, layout)
+    pc = packed_chunk_bytes(elems)
+    pool = torch.zeros(NB, 1, 2, pc, dtype=torch.uint8).pin_memory()
+    host = HostSide(pool.data_ptr(), 2 * pc, pc, 2 * pc, NB)
+    ids = np.arange(n, dtype=np.int64)
+    keep = kv_quant_fp8(reg, host, ids, ids, h2d=False)
+    torch.cuda.synchronize()
+    for t in kv:
+        t.fill_(1)
+    keep += kv_quant_fp8(reg, host, ids, ids, h2d=True)
+    torch.cuda.synchronize()
+    for k in range(2):
+        q, s = reference_pack(src[k])
+        assert torch.equal(pool[:, 0, k, :elems], q.cpu())
+        assert torch.equal(pool[:, 0, k, elems:].contiguous().view(torch.float32), s.cpu())
+        got = kv[0][k].reshape(NB, elems)
+        assert torch.equal(got.view(torch.int16), reference_unpack(q, s).view(torch.int16))
+        assert bool((got[src[k] == 0] == 0).all())
+
+
 @pytest.mark.parametrize("shape", [KVShape("l1", 16, 8, 128, tokens_per_block=16),
                                    KVShape("l2", 15, 1, 576, use_mla=True, tokens_per_block=64)])   # ragged last tile
 def test_copy_engine_route_moves_the_same_bytes(shape):
