@@ -106,6 +106,12 @@ def host_register_chunk_bytes() -> int:
     return int(gb * (1 << 30)) if gb > 0 else 0
 
 
+def host_pool_in_parts(host) -> bool:
+    """True when the pool is registered with CUDA in more than one part. Kernels address all of it; a driver copy must
+    not straddle two registrations."""
+    return 0 < host_register_chunk_bytes() < host.num_blocks * host.block_bytes
+
+
 class StorageEngine:
     def __init__(self, model_config: ModelConfig, cache_config: CacheConfig, cuda_register: Optional[bool] = None,
                  numa_node: int = -1) -> None:

@@ -12,15 +12,14 @@ from __future__ import annotations
 from typing import Any, Dict
 
 from ... import _native
-from ...storage.storage_engine import host_register_chunk_bytes
 
 
 def codec_link(worker: Any, staging_bytes: int):
     """The native router of a worker's ops between kernel and copy engines, or None where every op belongs to the
-    kernel: an engine of the user's choice (FLEXKV_TRANSFER_ENGINE), several ranks behind one op, whose slices of a
-    host block are not one span and whose launches read the same id arrays, or a host pool registered in parts, which
-    a driver copy must not straddle."""
-    if len(worker.regs) != 1 or not worker.copy_engines or host_register_chunk_bytes():
+    kernel: an engine of the user's choice (FLEXKV_TRANSFER_ENGINE) or a host pool registered in parts
+    (``worker.copy_engines``), or several ranks behind one op, whose slices of a host block are not one span and whose
+    launches read the same id arrays."""
+    if len(worker.regs) != 1 or not worker.copy_engines:
         return None
     reg = worker.regs[0]
     return _native.C.CodecLink(reg.device_id, reg.num_layers, reg.kv_dim, worker.kv_stride, staging_bytes)

@@ -26,8 +26,7 @@ from .. import _native
 from ..common.config import GLOBAL_CONFIG_FROM_ENV
 from ..common.debug import flexkv_logger
 from ..common.transfer import LayerwiseTransferOp, TransferOp, WorkerKey
-from ..storage.storage_engine import host_register_chunk_bytes
-from .workers import OpOutcome, TransferWorker, _launch_cfg
+from .workers import OpOutcome, TransferWorker, host_launch_cfg
 
 HEADER = struct.Struct("iiii")
 ACK = b"\x01"
@@ -165,11 +164,9 @@ def build_layerwise_group(storage, model_config, key: WorkerKey, notify_mode: Op
         layer_stride, kv_stride, tp_stride = host.layer_stride, host.kv_stride, host.chunk_bytes // n_slices
     host_d = dict(base=host.base, layer_stride=layer_stride, kv_stride=kv_stride, block_stride=host.block_bytes,
                   num_blocks=host.num_blocks)
-    h2d = _launch_cfg(env, True)
-    if host_register_chunk_bytes() and h2d["engine"] >= 2:
-        h2d["engine"] = 0           # a host pool registered in parts: driver copies must not straddle two of them
     opts = dict(num_layers=reg0.num_layers, kv_dim=reg0.kv_dim, chunk_bytes=reg0.chunk_bytes,
-                cpu_tp_stride=tp_stride, shared_kv=shared, h2d=h2d, d2h=_launch_cfg(env, False),
+                cpu_tp_stride=tp_stride, shared_kv=shared, h2d=host_launch_cfg(env, True, host),
+                d2h=host_launch_cfg(env, False, host),
                 max_blocks_per_op=max(4096, min(1 << 18, host.num_blocks)),
                 notify_mode=notify_mode or env.layerwise_notify_mode, num_counters=num_counters,
                 layers_per_batch=layers_per_batch, create_eventfds=create_eventfds)
@@ -233,8 +230,8 @@ def _build_multi_group(storage, model_config, key: WorkerKey, env, notify_mode, 
             options=dict(num_layers=g.num_layers, kv_dim=g.kv_dim, chunk_bytes=g.chunk_bytes,
                          cpu_tp_stride=0 if shared else slice_bytes, shared_kv=shared)))
     members = layer_members(model_config, lay.groups)
-    opts = dict(num_layers=len(members), kv_dim=1, chunk_bytes=16, h2d=_launch_cfg(env, True),
-                d2h=_launch_cfg(env, False), max_blocks_per_op=max(4096, min(1 << 18, host.num_blocks)),
+    opts = dict(num_layers=len(members), kv_dim=1, chunk_bytes=16, h2d=host_launch_cfg(env, True, host),
+                d2h=host_launch_cfg(env, False, host), max_blocks_per_op=max(4096, min(1 << 18, host.num_blocks)),
                 notify_mode=notify_mode or env.layerwise_notify_mode, num_counters=num_counters,
                 layers_per_batch=1, create_eventfds=create_eventfds)
     host_d = dict(base=host.base, layer_stride=host.block_bytes, kv_stride=0, block_stride=host.block_bytes,

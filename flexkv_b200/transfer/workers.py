@@ -24,6 +24,7 @@ from ..common.config import GLOBAL_CONFIG_FROM_ENV, CacheConfig, ModelConfig
 from ..common.debug import flexkv_logger
 from ..common.storage import KVCacheLayoutType
 from ..common.transfer import TransferOp, TransferType, WorkerKey
+from ..storage.storage_engine import host_pool_in_parts
 
 
 @dataclass
@@ -111,6 +112,14 @@ def _launch_cfg(env, h2d: bool) -> Dict[str, int]:
                 tile_bytes=env.transfer_tile_bytes, engine=engine)
 
 
+def host_launch_cfg(env, h2d: bool, host) -> Dict[str, int]:
+    """The engine for a host pool: one that is registered in parts belongs to the kernels."""
+    cfg = _launch_cfg(env, h2d)
+    if cfg["engine"] >= _ENGINE_IDS["ce"] and host_pool_in_parts(host):
+        cfg["engine"] = _ENGINE_IDS["tma"]
+    return cfg
+
+
 def build_transfer_group(storage, model_config: ModelConfig, key: WorkerKey, high_priority: bool = False,
                          max_blocks_per_op: Optional[int] = None):
     """One native TransferGroup over every registered rank of ``key``."""
@@ -144,7 +153,8 @@ def build_transfer_group(storage, model_config: ModelConfig, key: WorkerKey, hig
                   kv_stride=kv_stride, block_stride=host.block_bytes, num_blocks=host.num_blocks)
     opts = dict(num_layers=reg0.num_layers, kv_dim=reg0.kv_dim, chunk_bytes=reg0.chunk_bytes,
                 cpu_tp_stride=tp_stride, shared_kv=shared, shared_mode=env.kv_shared_across_ranks_mode,
-                h2d=_launch_cfg(env, True), d2h=_launch_cfg(env, False), high_priority_stream=high_priority,
+                h2d=host_launch_cfg(env, True, host), d2h=host_launch_cfg(env, False, host),
+                high_priority_stream=high_priority,
                 **({"ce_max_copies": int(os.environ["FLEXKV_CE_SEGMENT_THRESHOLD"])}
                    if os.environ.get("FLEXKV_CE_SEGMENT_THRESHOLD") else {}),
                 max_blocks_per_op=max_blocks_per_op or max(4096, min(1 << 18, host.num_blocks)))
@@ -366,7 +376,7 @@ class QuantGpuHostWorker(TransferWorker):
         self.host = host
         self.layer_stride, self.kv_stride, self.tp_stride = host.layer_stride // n, host.kv_stride // n, \
             host.block_bytes // n
-        self.copy_engines = _launch_cfg(GLOBAL_CONFIG_FROM_ENV, h2d)["engine"] >= _ENGINE_IDS["ce"]
+        self.copy_engines = host_launch_cfg(GLOBAL_CONFIG_FROM_ENV, h2d, host)["engine"] >= _ENGINE_IDS["ce"]
         self.strategy = build_compressors(host, self.layers_total, self.regs[0].kv_dim, len(self.regs), self.shared)
         self.strategy.attach(self)
         # Tile pipelines per launch (two share an SM in the lossless codec's kernel). Measured on B200 with
