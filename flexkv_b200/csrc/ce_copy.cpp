@@ -221,8 +221,26 @@ bool ce_plan_staged(const KvCopyParams& p, int64_t* g, int64_t* c, int64_t min_r
   return true;
 }
 
+namespace {
+
+// Leaves nothing in flight on either stream of an op that could not be queued as a whole (an error, an exception).
+struct SettleOnFailure {
+  const CeStaging& st;
+  cudaStream_t stream;
+  bool queued = false;
+  ~SettleOnFailure() {
+    if (queued) return;
+    (void)cudaStreamSynchronize(stream);
+    (void)cudaStreamSynchronize(st.copy_stream);
+    (void)cudaGetLastError();
+  }
+};
+
+}  // namespace
+
 cudaError_t ce_copy_staged(const KvCopyParams& p, const CeStagePlan& plan, CeStaging& st, const CeStageKernel& kernel,
                            cudaStream_t stream, const CeLinkCopy* link) {
+  SettleOnFailure settle{st, stream};
   const int64_t block_bytes = p.c_block_stride;
   cudaError_t e = cudaSuccess;
   auto by_kernel = [&](int64_t first, int64_t pairs) -> cudaError_t {
@@ -281,6 +299,7 @@ cudaError_t ce_copy_staged(const KvCopyParams& p, const CeStagePlan& plan, CeSta
   // the caller's stream ends after the last copies
   for (b = 0; b < kCeStageBufs && e == cudaSuccess; ++b)
     if (st.used[b]) e = cudaStreamWaitEvent(stream, st.copy_done[b], 0);
+  settle.queued = e == cudaSuccess;
   return e;
 }
 

@@ -124,7 +124,8 @@ struct CeLinkCopy {
 // Moves the op: pieces through the staging buffers, gather or scatter kernel on `stream`, large copies on the
 // staging's own stream, both buffers in flight; the other pairs by the kernel, on `stream`, beside the last copies
 // (offload) or the first ones (restore). When it returns, everything has been queued and `stream` waits for the last
-// copy. `p` carries the id arrays as planned.
+// copy; when it fails, part of the op may have been moved and nothing of it is in flight any more. `p` carries the id
+// arrays as planned.
 cudaError_t ce_copy_staged(const KvCopyParams& p, const CeStagePlan& plan, CeStaging& st, const CeStageKernel& kernel,
                            cudaStream_t stream, const CeLinkCopy* link = nullptr);
 

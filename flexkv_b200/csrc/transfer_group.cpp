@@ -198,7 +198,10 @@ int TransferGroup::retire_task(int r, const Launched& l, int slot, float& ms) {
   cudaError_t e = l.err;
   if (e == cudaSuccess) e = cudaEventSynchronize(rk.ev1[slot]);
   if (e != cudaSuccess) {
+    // part of the op may have been queued: it reads the op's ids and moves blocks until the stream has passed it
+    (void)cudaStreamSynchronize(rk.stream);
     (void)cudaGetLastError();
+    (void)collect_status(rk.status + slot * kStatusWords);
     return -(int)e;
   }
   cudaEventElapsedTime(&ms, rk.ev0[slot], rk.ev1[slot]);
