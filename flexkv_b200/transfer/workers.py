@@ -411,6 +411,14 @@ class QuantGpuHostWorker(TransferWorker):
     def close(self) -> None:
         self.strategy.detach()
 
+    def _settle(self) -> None:
+        """After an op that could not be launched on every rank: what was queued, on any of them, still reads the id
+        buffers and writes the status words that the next op will use."""
+        for st in self.streams.values():
+            st.synchronize()
+        for words in self._words.values():
+            words[:] = 0
+
     def execute(self, op: TransferOp) -> OpOutcome:
         torch = self._torch
         if self.h2d:
@@ -446,7 +454,7 @@ class QuantGpuHostWorker(TransferWorker):
                 try:
                     self.strategy.run(params, i, self.num_ctas, st.cuda_stream)
                 except Exception:
-                    st.synchronize()        # what was queued still reads the id buffers
+                    self._settle()
                     raise
                 e1.record(st)
             evs.append((e0, e1, reg.device_id))
