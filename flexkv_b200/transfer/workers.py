@@ -390,21 +390,21 @@ class QuantGpuHostWorker(TransferWorker):
         self._torch = torch
         self.streams = {r.device_id: torch.cuda.Stream(device=r.device_id) for r in self.regs}
         # Kept between ops, which this worker runs one at a time: pinned id buffers and status words that the kernels
-        # address themselves, and a pair of events per device.
+        # address themselves, and a pair of events per rank (ranks may share a device and its stream).
         self._ids = torch.empty((2, 4096), dtype=torch.int64).pin_memory()
         self.status = {r.device_id: torch.zeros(8, dtype=torch.int32).pin_memory() for r in self.regs}
         self._words = {d: t.numpy() for d, t in self.status.items()}
-        self._events = {}
+        self._events = []
         for r in self.regs:
             with torch.cuda.device(r.device_id):
                 _native.C.codec_load_kernels()
-                self._events[r.device_id] = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
+                self._events.append((torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)))
 
     def warm_thread(self) -> None:
-        for d, (e0, e1) in self._events.items():
-            with self._torch.cuda.device(d):
-                e0.record(self.streams[d])
-                e1.record(self.streams[d])
+        for r, (e0, e1) in zip(self.regs, self._events):
+            with self._torch.cuda.device(r.device_id):
+                e0.record(self.streams[r.device_id])
+                e1.record(self.streams[r.device_id])
                 e1.synchronize()
                 e0.elapsed_time(e1)
 
@@ -448,7 +448,7 @@ class QuantGpuHostWorker(TransferWorker):
                           gpu_num_blocks=reg.num_blocks, cpu_num_blocks=self.host.num_blocks,
                           status_ptr=self.status[reg.device_id].data_ptr(), h2d=int(self.h2d))
             st = self.streams[reg.device_id]
-            e0, e1 = self._events[reg.device_id]
+            e0, e1 = self._events[i]
             with torch.cuda.device(reg.device_id):
                 e0.record(st)
                 try:

@@ -51,7 +51,7 @@ def _worker(devices, run, shared=False):
     w._ids = torch.zeros((2, 64), dtype=torch.int64)
     w.status = {d: torch.zeros(8, dtype=torch.int32) for d in devices}
     w._words = {d: t.numpy() for d, t in w.status.items()}
-    w._events = {d: (Event(clock, log), Event(clock, log)) for d in devices}
+    w._events = [(Event(clock, log), Event(clock, log)) for _ in devices]
 
     class Strategy:
         def run(self, params, rank, num_ctas, stream):
@@ -77,3 +77,10 @@ def test_a_rank_that_cannot_launch_waits_for_the_others():
         w.execute(_op())
     assert {e for e in log if e[0] == "sync"} == {("sync", 0), ("sync", 1), ("sync", 2)}
     assert not any(words.any() for words in w._words.values())
+
+@pytest.mark.parametrize("devices", [[0], [0, 1], [0, 0, 0]])
+def test_time_of_an_op_is_that_of_its_slowest_rank(devices):
+    took = [7, 3, 2]
+    w, _ = _worker(devices, lambda rank, w: took[rank])
+    out = w.execute(_op())
+    assert out.success and out.gpu_ms == 7.0
