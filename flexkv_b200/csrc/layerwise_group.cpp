@@ -421,6 +421,14 @@ cudaError_t LayerwiseGroup::queue_staged(int r, const Job& j, const int64_t* gpu
   return e;
 }
 
+// Before a restore that could not be queued as a whole is reported: what was queued of it still reads its block ids and
+// writes pages, status words and flags.
+void LayerwiseGroup::settle(Rank& rk) {
+  (void)cudaStreamSynchronize(rk.stream);
+  if (rk.staging.copy_stream) (void)cudaStreamSynchronize(rk.staging.copy_stream);
+  (void)collect_status(rk.status);
+}
+
 // Multi-group restore of one rank: model layer by model layer, one launch per member; the last
 // member's launch carries the completion signal of the model layer (same stream, so the earlier
 // members have landed when its last CTA publishes the flag).
@@ -499,6 +507,7 @@ void LayerwiseGroup::run_job_members(int r, const Job& j) {
   if (err == cudaSuccess) err = cudaStreamSynchronize(rk.stream);
   if (err == cudaSuccess) err = cudaStreamSynchronize(rk.notify_stream);
   if (err != cudaSuccess) {
+    if (err != cudaErrorTimeout) settle(rk);
     (void)cudaGetLastError();
     (void)cudaStreamSynchronize(rk.notify_stream);   // callbacks already queued run first
     (void)cudaGetLastError();
@@ -627,6 +636,7 @@ void LayerwiseGroup::run_job(int r, const Job& j) {
   if (err == cudaSuccess) err = cudaStreamSynchronize(rk.stream);
   if (err == cudaSuccess) err = cudaStreamSynchronize(rk.notify_stream);
   if (err != cudaSuccess) {
+    if (err != cudaErrorTimeout) settle(rk);
     (void)cudaGetLastError();
     (void)cudaStreamSynchronize(rk.notify_stream);   // callbacks already queued run first
     (void)cudaGetLastError();

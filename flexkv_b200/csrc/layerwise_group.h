@@ -176,6 +176,7 @@ class LayerwiseGroup {
   bool plan_staged(Rank& rk, const Job& j, const KvCopyParams& p, std::vector<CeHostRun>& runs);
   cudaError_t queue_staged(int r, const Job& j, const int64_t* gpu_ids, const std::vector<CeHostRun>& runs);
   cudaError_t stage_ids(Rank& rk, const Job& j, const int64_t*& gpu_ids, const int64_t*& cpu_ids);
+  static void settle(Rank& rk);
   void notify(int rank, int counter, int layer_lo, int layer_hi);
   // failure path of a job: records the status for counter_status(), then publishes the epoch to the flags of
   // layers [from_layer, L) from the host and fires their eventfds (one unit each, as for a good layer: the

@@ -131,6 +131,8 @@ cudaError_t launch_kv_copy(const KvCopyParams& p, const KvCopyLaunch&, cudaStrea
     if (const int err = host_kv_copy(p, 1))
       for (int b = 0; b < kStatusWords; ++b)
         if (err & (1 << b)) p.status[b] = 1;
+    if (p.done_counter)
+      for (int l = p.layer_start; l < p.layer_start + p.num_layers; ++l) p.dev_flags[l] = p.host_flags[l] = p.epoch;
   });
   return cudaSuccess;
 }

@@ -28,3 +28,7 @@ TRANSFER = ("transfer_group.cpp", "ce_copy.cpp", "ptr_table.cpp", "kv_copy_host.
 
 def test_failed_launch_leaves_nothing_in_flight(tmp_path):
     _run(tmp_path, "failed_launch", TRANSFER)
+
+
+def test_failed_layerwise_restore_leaves_nothing_in_flight(tmp_path):
+    _run(tmp_path, "failed_layerwise", ("layerwise_group.cpp",) + TRANSFER)
