@@ -224,7 +224,8 @@ kv_copy_bulk_kernel(const __grid_constant__ KvCopyParams p, int tile_bytes, int 
         }
       }
     }
-    dead = __shfl_sync(0xffffffffu, dead, 0);   // also orders lane 0's reads before the next batch is written
+    __syncwarp();     // lane 0 has read its descriptors before the next batch is written over the oldest of them
+    dead = __shfl_sync(0xffffffffu, dead, 0);
     if (dead) break;
   }
   err = (int)__reduce_or_sync(0xffffffffu, (unsigned)err);
