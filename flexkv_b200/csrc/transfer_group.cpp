@@ -133,7 +133,8 @@ void TransferGroup::fill_params(int r, const Task& t, KvCopyParams& p, bool& ski
                  t.num_layers, t.rotate, p, skip);
 }
 
-// Queues one op of rank `r` on its stream, with the events and status words of `slot`. Called with the rank's exec_mu.
+// Queues one op of rank `r` on its stream, with the events and status words of `slot`. The caller has set the rank's
+// `busy`.
 TransferGroup::Launched TransferGroup::launch_task(int r, const Task& t, int slot) {
   Rank& rk = *ranks_[(size_t)r];
   Launched l;
@@ -248,15 +249,16 @@ void TransferGroup::rank_main(int r) {
     batch.clear();
     {
       std::unique_lock<std::mutex> lk(rk.mu);
-      rk.cv.wait(lk, [&] { return stop_.load() || !rk.q.empty(); });
+      rk.busy = false;
+      rk.cv.wait(lk, [&] { return (stop_.load() || !rk.q.empty()) && !rk.busy; });
       if (rk.q.empty() && stop_.load()) break;
       while (!rk.q.empty() && (int)batch.size() < kInflight) {
         batch.push_back(rk.q.front());
         rk.q.pop_front();
       }
+      rk.busy = true;
     }
     // launch everything that is queued, then retire in order: consecutive ops overlap their launch latency
-    std::lock_guard<std::mutex> exec(rk.exec_mu);
     Launched l[kInflight];
     for (size_t i = 0; i < batch.size(); ++i) l[i] = launch_task(r, batch[i], (int)i);
     for (size_t i = 0; i < batch.size(); ++i) {
@@ -336,20 +338,40 @@ OpResult TransferGroup::transfer(const int64_t* gpu_blocks, const int64_t* cpu_b
     return wait(submit(gpu_blocks, cpu_blocks, n, h2d, layer_start, num_layers, engine_override));
   const Task t = make_task(gpu_blocks, cpu_blocks, n, h2d, layer_start, num_layers, engine_override);
   Rank& rk = *ranks_[0];
+  bool here;
+  {
+    std::lock_guard<std::mutex> g(rk.mu);
+    here = rk.q.empty() && !rk.busy;
+    if (here) rk.busy = true;
+    else rk.q.push_back(t);
+  }
+  if (!here) {                            // behind the ops in front of it, and launched ahead with those beside it
+    rk.cv.notify_one();
+    return wait(t.ticket);
+  }
+  auto leave = [&] {
+    bool more;
+    {
+      std::lock_guard<std::mutex> g(rk.mu);
+      rk.busy = false;
+      more = !rk.q.empty() || stop_.load();
+    }
+    if (more) rk.cv.notify_one();
+  };
   int before = -1;
   if (cudaGetDevice(&before) != cudaSuccess) before = -1;
   int status = -(int)cudaErrorUnknown;
   float ms = 0.f;
   try {
-    // behind what the rank's thread has in hand; it takes nothing new meanwhile
-    std::lock_guard<std::mutex> exec(rk.exec_mu);
     const cudaError_t e = before == gpus_[0].device ? cudaSuccess : cudaSetDevice(gpus_[0].device);
     status = e == cudaSuccess ? retire_task(0, launch_task(0, t, 0), 0, ms) : -(int)e;
   } catch (...) {
+    leave();
     finish(t.ticket, status, 0.f);      // gives the id ring slot back
     wait(t.ticket);
     throw;
   }
+  leave();
   finish(t.ticket, status, ms);
   if (before >= 0 && before != gpus_[0].device) cudaSetDevice(before);
   return wait(t.ticket);

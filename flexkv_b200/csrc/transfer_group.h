@@ -86,8 +86,8 @@ class TransferGroup {
                   int num_layers, int engine_override = -1);
   OpResult wait(uint64_t ticket);
   bool poll(uint64_t ticket);
-  // Blocking. With one rank the op is launched and waited for on the calling thread: handing it to the rank's thread
-  // and being woken by it cost a 2 MiB op some 40 us.
+  // Blocking. With one rank that has nothing else to do the op is launched and waited for on the calling thread: handing
+  // it to the rank's thread and being woken by it cost a 2 MiB op some 40 us.
   OpResult transfer(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d, int layer_start,
                     int num_layers, int engine_override = -1);
   // Makes the first rank's device the calling thread's, as a thread that will call transfer() does once.
@@ -124,7 +124,7 @@ class TransferGroup {
     std::condition_variable cv;
     std::deque<Task> q;
     cudaStream_t stream = nullptr;
-    std::mutex exec_mu;         // held from the first launch of a batch of ops to the retirement of its last
+    bool busy = false;          // guarded by mu: a thread is launching or retiring ops of this rank
     cudaEvent_t ev0[kInflight] = {}, ev1[kInflight] = {};
     int32_t* status = nullptr;  // mapped pinned words, kStatusWords for each op in flight
     CeStaging staging;          // device staging of the gather + large-copy route

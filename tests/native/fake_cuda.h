@@ -31,7 +31,7 @@ inline uint64_t next_id = 1;
 inline std::map<cudaStream_t, std::deque<Op>> streams;
 inline std::map<cudaEvent_t, Mark> marks;
 inline std::atomic<int> launches{0}, fail_launch{-1};   // the launch of this number fails
-inline std::atomic<int> max_queued{0};                  // kernels of one stream queued at a time, at most
+inline std::function<void(const fkv::KvCopyParams&)> on_launch;   // on the launching thread, before a launch
 
 inline void drain(cudaStream_t s, uint64_t upto) {
   auto& q = streams[s];
@@ -126,6 +126,7 @@ namespace fkv {
 
 cudaError_t kv_copy_load_kernels() { return cudaSuccess; }
 cudaError_t launch_kv_copy(const KvCopyParams& p, const KvCopyLaunch&, cudaStream_t s) {
+  if (fake::on_launch) fake::on_launch(p);
   if (fake::launches++ == fake::fail_launch) return cudaErrorLaunchOutOfResources;
   fake::push(s, [p] {
     if (const int err = host_kv_copy(p, 1))

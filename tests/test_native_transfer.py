@@ -32,3 +32,7 @@ def test_failed_launch_leaves_nothing_in_flight(tmp_path):
 
 def test_failed_layerwise_restore_leaves_nothing_in_flight(tmp_path):
     _run(tmp_path, "failed_layerwise", ("layerwise_group.cpp",) + TRANSFER)
+
+
+def test_threads_share_a_group(tmp_path):
+    _run(tmp_path, "shared_group", TRANSFER)
