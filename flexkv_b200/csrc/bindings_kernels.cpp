@@ -148,7 +148,10 @@ void init_kernel_bindings(py::module_& m) {
         throw_on(e, "kv_compress_bf16");
       }, py::arg("params"), py::arg("size_table_ptr"), py::arg("layers_total"), py::arg("num_ctas"),
          py::arg("staged_ctas"), py::arg("stream"))
-      .def_property_readonly("staged_ops", &CodecLink::staged_ops);
+      .def_property_readonly("staged_ops", &CodecLink::staged_ops)
+      .def_property_readonly_static("MIN_QUANT_BYTES", [](py::object) { return CodecLink::kMinQuantBytes; })
+      .def_property_readonly_static("MIN_ROW_BYTES", [](py::object) { return CodecLink::kMinRowBytes; })
+      .def_property_readonly_static("MIN_ROW_CHUNK", [](py::object) { return CodecLink::kMinRowChunk; });
   m.def("fp8_packed_chunk_bytes", &fp8_packed_chunk_bytes);
 
   m.def("kv_compress_bf16", [](py::dict params, uint64_t size_table_ptr, int layers_total, int num_ctas,

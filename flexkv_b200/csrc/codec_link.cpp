@@ -22,11 +22,6 @@ class DeviceScope {
 }  // namespace
 
 namespace {
-// Ops of fewer host bytes stay with the kernel, whose start and end are shorter. B200, us, kernel -> staged: fp8 out
-// 483 (25 MB) -> 483, 944 (50 MB) -> 910, 5025 (268 MB) -> 4707; lossless in, llama3-8b pages 885 (66 MB of slots)
-// -> 873, 3451 (258 MB) -> 3305, 6858 -> 6538, deepseek-v3 pages 893 (64 MB) -> 931, 1751 (127 MB) -> 1750,
-// 3430 (254 MB) -> 3382.
-constexpr int64_t kMinQuantBytes = 48 << 20, kMinRowBytes = 128 << 20;
 // Slot bytes of the last piece of a restore: smaller ones come in copies too short for the link.
 constexpr int64_t kRowRampBytes = 12 << 20;
 }  // namespace
@@ -118,8 +113,7 @@ bool plan_rows(const KvCopyParams& p, const uint32_t* sizes, const CeHostRun& pi
 cudaError_t CodecLink::compress_bf16(const KvCopyParams& p, uint32_t* size_table, int layers_total, int num_ctas,
                                      int staged_ctas, cudaStream_t stream) {
   CeStagePlan pl;
-  // rows of chunks below 4096 values are too short for a copy engine: 48.2 GB/s at 2048 values, the kernel 50.4
-  if (!p.h2d || size_table == nullptr || p.chunk_bytes < 8192 || p.chunk_bytes % 2048 != 0 || layers_total != num_layers_ ||
+  if (!p.h2d || size_table == nullptr || p.chunk_bytes < kMinRowChunk || p.chunk_bytes % 2048 != 0 || layers_total != num_layers_ ||
       !plan(p, kMinRowBytes, kRowRampBytes, pl))
     return launch_kv_compress_bf16(p, size_table, layers_total, num_ctas, stream);
   ++staged_ops_;

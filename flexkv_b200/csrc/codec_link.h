@@ -15,9 +15,17 @@
 
 namespace fkv {
 
-// One GPU, one direction. run() is called by one thread at a time.
+// One GPU, one direction. quant_fp8() or compress_bf16() is called by one thread at a time.
 class CodecLink {
  public:
+  // Ops of fewer host bytes stay with the kernel, whose start and end are shorter. B200, us, kernel -> staged: fp8 out
+  // 483 (25 MB) -> 483, 944 (50 MB) -> 910, 5025 (268 MB) -> 4707; lossless in, llama3-8b pages 885 (66 MB of slots)
+  // -> 873, 3451 (258 MB) -> 3305, 6858 -> 6538, deepseek-v3 pages 893 (64 MB) -> 931, 1751 (127 MB) -> 1750,
+  // 3430 (254 MB) -> 3382.
+  static constexpr int64_t kMinQuantBytes = 48 << 20, kMinRowBytes = 128 << 20;
+  // Rows of smaller chunks (bf16 bytes) are too short for a copy engine: 48.2 GB/s at 2048 values, the kernel 50.4.
+  static constexpr int64_t kMinRowChunk = 8192;
+
   // `chunk_slot`: bytes a packed (layer, kv, block) chunk takes in the host pool; `staging_bytes` of each of the two
   // staging buffers.
   CodecLink(int device, int num_layers, int kv_dim, int64_t chunk_slot, int64_t staging_bytes = kCeStageBytes);

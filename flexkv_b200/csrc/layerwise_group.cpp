@@ -79,13 +79,26 @@ LayerwiseGroup::LayerwiseGroup(std::vector<LayerwiseMemberGroup> groups, std::ve
   start_ranks();
 }
 
+// One layer per copy and scatter. B200, GB/s: rows of 64 KiB come in at 54.7 (50.3 where a copy has 32 of them), rows of
+// 8 KiB at 48.7, the layer-major kernel reads 51; a copy costs 3.5 us beside its bytes.
+constexpr int64_t kLayerMinBytes = 6 << 20, kLayerMinRowBytes = 16 << 10, kLayerMinRunBytes = 2 << 20;
+
+// Whether the geometry of the pool and the largest job allow the copy-engine form at all.
+static bool rows_fit(const GroupOptions& g, const HostSide& host) {
+  const int64_t row = g.chunk_bytes * g.kv_dim;
+  const int64_t blocks = host.num_blocks > 0 ? std::min(host.num_blocks, g.max_blocks_per_op) : g.max_blocks_per_op;
+  return (g.kv_dim == 1 || host.kv_stride == g.chunk_bytes) && host.block_stride >= row && row >= kLayerMinRowBytes &&
+         row * blocks >= kLayerMinBytes;
+}
+
 void LayerwiseGroup::start_ranks() {
   if (gpus_.empty()) throw std::invalid_argument("LayerwiseGroup: no GPUs");
   if (opt_.num_counters < 1 || opt_.layers_per_batch < -1) throw std::invalid_argument("LayerwiseGroup: bad options");
   const int L = opt_.group.num_layers, R = (int)gpus_.size(), C = opt_.num_counters;
   if (opt_.group.h2d.engine >= kEngineCe) {      // names of the router, which the kernel launcher does not know
     opt_.group.h2d.engine = kEngineTma;
-    copy_engines_ = mgroups_.empty() && opt_.size_table == nullptr && opt_.layers_per_batch < 0;
+    copy_engines_ = mgroups_.empty() && opt_.size_table == nullptr && opt_.layers_per_batch < 0 &&
+                    rows_fit(opt_.group, host_);
   }
   epochs_.assign((size_t)C, 0);
   reserved_.assign((size_t)C, 0);
@@ -349,15 +362,9 @@ cudaError_t LayerwiseGroup::stage_ids(Rank& rk, const Job& j, const int64_t*& gp
   return err;
 }
 
-// One layer per copy and scatter. B200, GB/s: rows of 64 KiB come in at 54.7 (50.3 where a copy has 32 of them), rows of
-// 8 KiB at 48.7, the layer-major kernel reads 51; a copy costs 3.5 us beside its bytes.
-constexpr int64_t kLayerMinBytes = 6 << 20, kLayerMinRowBytes = 16 << 10, kLayerMinRunBytes = 2 << 20;
-
 bool LayerwiseGroup::plan_staged(Rank& rk, const Job& j, const KvCopyParams& p, std::vector<CeHostRun>& runs) {
   const int64_t row = p.chunk_bytes * p.kv_dim, layer = row * j.n;
-  if (!copy_engines_ || p.c_use_table || (p.kv_dim > 1 && p.c_kv_stride != p.chunk_bytes) || p.c_block_stride < row ||
-      row < kLayerMinRowBytes || layer < kLayerMinBytes || rk.staging.block_bytes != row || !kv_copy_tables_ok(p))
-    return false;
+  if (!copy_engines_ || layer < kLayerMinBytes || rk.staging.block_bytes != row || !kv_copy_tables_ok(p)) return false;
   runs.clear();
   for (int64_t i = 0; i < j.n; ++i) {
     const int64_t g = j.gpu_blocks[i], c = j.cpu_blocks[i];

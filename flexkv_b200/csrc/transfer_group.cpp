@@ -229,7 +229,8 @@ void TransferGroup::rank_main(int r) {
     // the staging buffers are in place before the first op (allocated by it, they cost it 10 to 16 ms)
     auto may_stage = [](const KvCopyLaunch& c) { return c.engine == kEngineCe || c.engine == kEngineAuto; };
     if (gpus_.size() == 1 && opt_.ce_staging_blocks != 0 && (may_stage(opt_.h2d) || may_stage(opt_.d2h)) &&
-        host_.block_stride == opt_.chunk_bytes * opt_.kv_dim * opt_.num_layers)
+        host_.block_stride == opt_.chunk_bytes * opt_.kv_dim * opt_.num_layers &&
+        host_.num_blocks * host_.block_stride >= opt_.ce_policy.min_bytes_per_copy)
       ce_staging_prepare(rk.staging, std::max<int64_t>(0, opt_.ce_staging_blocks), host_.block_stride);
   } catch (const std::exception& e) {
     std::lock_guard<std::mutex> g(rk.mu);

@@ -14,14 +14,18 @@ from typing import Any, Dict
 from ... import _native
 
 
-def codec_link(worker: Any, staging_bytes: int):
+def codec_link(worker: Any, staging_bytes: int, min_op_bytes: int, min_chunk: int = 0):
     """The native router of a worker's ops between kernel and copy engines, or None where every op belongs to the
     kernel: an engine of the user's choice (FLEXKV_TRANSFER_ENGINE) or a host pool registered in parts
-    (``worker.copy_engines``), or several ranks behind one op, whose slices of a host block are not one span and whose
-    launches read the same id arrays."""
+    (``worker.copy_engines``), several ranks behind one op or one rank's slice of a wider block, which is not one span,
+    chunks below ``min_chunk`` bytes, or a pool that cannot hold an op of ``min_op_bytes``. The router takes twice
+    ``staging_bytes`` of GPU memory for its lifetime."""
     if len(worker.regs) != 1 or not worker.copy_engines:
         return None
-    reg = worker.regs[0]
+    reg, host = worker.regs[0], worker.host
+    if worker.kv_stride * reg.kv_dim * reg.num_layers != host.block_bytes or reg.chunk_bytes < min_chunk or \
+            host.num_blocks * host.block_bytes < min_op_bytes:
+        return None
     return _native.C.CodecLink(reg.device_id, reg.num_layers, reg.kv_dim, worker.kv_stride, staging_bytes)
 
 
@@ -75,7 +79,7 @@ class Fp8BlockScaleStrategy(CompressionStrategy):
 
     def attach(self, worker) -> None:
         super().attach(worker)
-        self._link = codec_link(worker, 32 << 20)
+        self._link = codec_link(worker, 32 << 20, _native.C.CodecLink.MIN_QUANT_BYTES)
 
     def detach(self) -> None:
         self._link = None
@@ -102,7 +106,8 @@ class ExponentPackStrategy(CompressionStrategy):
     def attach(self, worker) -> None:
         super().attach(worker)
         # restores only; rows of about 1000 tiles per copy need a larger buffer than whole blocks do
-        self._link = codec_link(worker, 64 << 20) if worker.h2d else None
+        C = _native.C.CodecLink
+        self._link = codec_link(worker, 64 << 20, C.MIN_ROW_BYTES, C.MIN_ROW_CHUNK) if worker.h2d else None
 
     def detach(self) -> None:
         self._link = None

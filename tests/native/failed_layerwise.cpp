@@ -1,27 +1,11 @@
 // A layerwise restore that fails half way leaves nothing in flight when its waiters are released.
 #include "fake_cuda.h"
+#include "fake_layerwise.h"
 
 #include <cstdio>
 #include <vector>
 
-#include "layerwise_group.h"
-
 using namespace fkv;
-
-extern "C" {
-cudaError_t cudaGetDriverEntryPoint(const char*, void**, unsigned long long, cudaDriverEntryPointQueryResult*) {
-  return cudaErrorNotSupported;
-}
-cudaError_t cudaLaunchHostFunc(cudaStream_t s, cudaHostFn_t fn, void* arg) {
-  fake::push(s, [=] { fn(arg); });
-  return cudaSuccess;
-}
-}
-namespace fkv {
-cudaError_t launch_kv_compress_bf16(const KvCopyParams&, uint32_t*, int, int, cudaStream_t) { return cudaErrorNotSupported; }
-int64_t SsdIoEngine::transfer(uint8_t*, const int64_t*, const int64_t*, int64_t n, bool, const SsdLayout&, int, int,
-                              uint8_t*) { return n; }
-}  // namespace fkv
 
 #define CHECK(c)                                                       \
   do {                                                                 \

@@ -31,6 +31,7 @@ inline uint64_t next_id = 1;
 inline std::map<cudaStream_t, std::deque<Op>> streams;
 inline std::map<cudaEvent_t, Mark> marks;
 inline std::atomic<int> launches{0}, fail_launch{-1};   // the launch of this number fails
+inline std::atomic<size_t> device_bytes{0};             // asked for with cudaMalloc so far
 inline std::function<void(const fkv::KvCopyParams&)> on_launch;   // on the launching thread, before a launch
 
 inline void drain(cudaStream_t s, uint64_t upto) {
@@ -63,7 +64,11 @@ cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
 cudaError_t cudaDeviceGetStreamPriorityRange(int* lo, int* hi) { *lo = *hi = 0; return cudaSuccess; }
-cudaError_t cudaMalloc(void** p, size_t n) { *p = std::malloc(n ? n : 1); return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) {
+  fake::device_bytes += n;
+  *p = std::malloc(n ? n : 1);
+  return cudaSuccess;
+}
 cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::malloc(n ? n : 1); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }

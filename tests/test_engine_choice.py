@@ -10,6 +10,7 @@ from flexkv_b200.transfer import layerwise, workers
 from flexkv_b200.transfer.compression import strategy
 
 MB = 1 << 20
+REAL = _native.C
 
 
 class Built(Exception):
@@ -60,6 +61,35 @@ def test_pool_registered_in_parts_is_left_to_the_kernels(native, monkeypatch, en
     for opts in (raw.value.args[0], layered.value.args[0]):
         assert opts["h2d"]["engine"] == opts["d2h"]["engine"] == want
     cfg = workers.host_launch_cfg(workers.GLOBAL_CONFIG_FROM_ENV, True, st.host)
-    worker = types.SimpleNamespace(regs=[st.gpu_regs[key][0]], copy_engines=cfg["engine"] >= 2, kv_stride=MB // 4)
-    if not worker.copy_engines:
-        assert strategy.codec_link(worker, 32 * MB) is None
+    assert cfg["engine"] == want
+
+
+@pytest.mark.parametrize("name,h2d,blocks,block_bytes,n_ranks,slice_of,want", [
+    ("fp8", True, 64, 2 * MB, 1, 1, True), ("fp8", False, 64, 2 * MB, 1, 1, True),
+    ("fp8", True, 23, 2 * MB, 1, 1, False),                    # a pool of 46 MiB: no op reaches the 48 MiB
+    ("fp8", True, 64, 2 * MB, 2, 1, False), ("fp8", True, 64, 2 * MB, 1, 2, False),
+    ("xp", True, 64, 2 * MB, 1, 1, True), ("xp", False, 64, 2 * MB, 1, 1, False),
+    ("xp", True, 63, 2 * MB, 1, 1, False),                     # 126 of 128 MiB
+    ("xp", True, 4096, 64 << 10, 1, 1, True), ("xp", True, 4096, 32 << 10, 1, 1, False)])       # 8 and 4 KiB chunks
+def test_codec_routers_are_made_where_they_can_be_used(native, name, h2d, blocks, block_bytes, n_ranks, slice_of, want):
+    """A router holds staging buffers on the GPU from its start."""
+    made = []
+
+    class CodecLink:
+        MIN_QUANT_BYTES, MIN_ROW_BYTES, MIN_ROW_CHUNK = (getattr(REAL.CodecLink, k) for k in (
+            "MIN_QUANT_BYTES", "MIN_ROW_BYTES", "MIN_ROW_CHUNK"))
+
+        def __init__(self, *args):
+            made.append(args)
+
+    _native.C.CodecLink = CodecLink
+    st = _storage(blocks, block_bytes)
+    reg = st.gpu_regs["k"][0]
+    worker = types.SimpleNamespace(regs=[reg] * n_ranks, copy_engines=True, h2d=h2d, host=st.host,
+                                   kv_stride=st.host.kv_stride // slice_of)
+    s = strategy.Fp8BlockScaleStrategy() if name == "fp8" else strategy.ExponentPackStrategy(object(), object())
+    s.attach(worker)
+    assert bool(made) == (s._link is not None) == want
+    worker.copy_engines = False
+    s.attach(worker)
+    assert s._link is None

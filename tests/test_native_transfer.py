@@ -36,3 +36,7 @@ def test_failed_layerwise_restore_leaves_nothing_in_flight(tmp_path):
 
 def test_threads_share_a_group(tmp_path):
     _run(tmp_path, "shared_group", TRANSFER)
+
+
+def test_staging_memory_is_taken_only_where_it_can_be_used(tmp_path):
+    _run(tmp_path, "device_memory", ("layerwise_group.cpp",) + TRANSFER)
