@@ -74,6 +74,7 @@ void init_layerwise_bindings(py::module_& m) {
       .def("update_gpu_ptrs", &LayerwiseGroup::update_gpu_ptrs)
       .def("update_group_gpu_ptrs", &LayerwiseGroup::update_group_gpu_ptrs)
       .def_property_readonly("is_multi_group", &LayerwiseGroup::multi_group)
+      .def_property_readonly("staged_restores", &LayerwiseGroup::staged_restores)
       .def("restore", [](LayerwiseGroup& g, I64Array gpu_blocks, I64Array cpu_blocks, int counter_id, py::object ssd,
                          py::object ssd_layout, py::object ssd_src, py::object cpu_dst) {
              if (gpu_blocks.size() != cpu_blocks.size()) throw std::invalid_argument("block id arrays differ in size");

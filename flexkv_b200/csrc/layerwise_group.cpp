@@ -575,6 +575,7 @@ void LayerwiseGroup::run_job(int r, const Job& j) {
     bool skip = false;
     fill_kv_params(gpus_[(size_t)r], host_, opt_.group, r, R, gpu_ids, cpu_ids, j.n, true, 0, L, 0, p, skip);
     staged = plan_staged(rk, j, p, runs);
+    if (staged && r == 0) staged_restores_.fetch_add(1, std::memory_order_relaxed);
     if (staged) err = queue_staged(r, j, gpu_ids, runs);
   }
   for (int b = 0; b < batches && !staged && err == cudaSuccess; ++b) {

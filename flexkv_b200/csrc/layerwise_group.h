@@ -120,6 +120,7 @@ class LayerwiseGroup {
   cudaError_t stream_wait_layer(int rank, int counter, int layer, cudaStream_t stream, uint32_t epoch = 0);
   // 0 while the newest restore on `counter` is running or has succeeded, else its failure status
   int counter_status(int counter) const { return counter_status_[(size_t)counter].load(std::memory_order_acquire); }
+  uint64_t staged_restores() const { return staged_restores_.load(); }   // that took the copy-engine form (first rank)
   int num_ranks() const { return (int)gpus_.size(); }
   // new tensor addresses after the engine re-created its cache; call with no restore in flight
   void update_gpu_ptrs(int rank, const std::vector<uint64_t>& ptrs);
@@ -191,6 +192,7 @@ class LayerwiseGroup {
   std::vector<std::vector<LayerMember>> members_;        // [model layer]
   LayerwiseOptions opt_;
   bool copy_engines_ = false;       // the engine option leaves the choice between kernels and copy engines to us
+  std::atomic<uint64_t> staged_restores_{0};
   std::vector<std::unique_ptr<Rank>> ranks_;
   std::atomic<bool> stop_{false};
   std::vector<int> eventfds_;       // [counters][ranks][layers]

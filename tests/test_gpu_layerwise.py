@@ -298,6 +298,31 @@ def test_layers_through_the_copy_engines_carry_the_same_bytes_and_signals(n, use
         for l in range(L):
             assert torch.equal(kv[l][d] if use_mla else kv[l][:, d], want[l])
             assert int((kv[l] != 0).any(-1).sum()) == int((want[l] != 0).any(-1).sum())     # nothing beside the pages
+    assert grp.staged_restores == 2
     bad = dst.copy()
     bad[3] = NB
-    assert grp.restore(bad, cpu, 1).status == 1
+    assert grp.restore(bad, cpu, 1).status == 1 and grp.staged_restores == 2
+
+
+@pytest.mark.parametrize("head_size,n,runs,staged", [(128, 96, 1, 1), (128, 95, 1, 0),      # 6 MiB a layer
+                                                     (128, 96, 3, 1), (128, 96, 4, 0),      # 2 MiB a run on average
+                                                     (32, 400, 1, 1), (16, 800, 1, 0)])     # rows of 16 KiB and of 8
+def test_which_restores_take_the_copy_engines(head_size, n, runs, staged):
+    shape = KVShape("lt", 2, 8, head_size, tokens_per_block=16)
+    NB = n + 8
+    kv, reg, pool, _, xfer = _setup(shape, NB=NB)
+    L, K, chunk = shape.num_layers, shape.kv_dim, reg.chunk_bytes
+    grp = C.LayerwiseGroup([reg.as_native()], dict(base=pool.data_ptr(), layer_stride=K * chunk, kv_stride=chunk,
+                                                   block_stride=L * K * chunk, num_blocks=NB),
+                           dict(num_layers=L, kv_dim=K, chunk_bytes=chunk, max_blocks_per_op=NB, notify_mode="polling",
+                                layers_per_batch=-1, h2d=dict(num_ctas=8, tile_bytes=16384, engine=3)))
+    cpu = np.concatenate([part + i for i, part in enumerate(np.array_split(np.arange(n), runs))]).astype(np.int64)
+    src = np.random.default_rng(4).permutation(NB)[:n].astype(np.int64)
+    assert xfer.transfer(src, cpu, False, 0, L, 0).status == 0
+    s = torch.from_numpy(src).cuda()
+    want = [t[:, s].clone() for t in kv]
+    for t in kv:
+        t.zero_()
+    assert grp.restore(src, cpu, 0).status == 0 and grp.staged_restores == staged
+    for l in range(L):
+        assert torch.equal(kv[l][:, s], want[l])
