@@ -113,6 +113,7 @@ bool plan_rows(const KvCopyParams& p, const uint32_t* sizes, const CeHostRun& pi
 cudaError_t CodecLink::compress_bf16(const KvCopyParams& p, uint32_t* size_table, int layers_total, int num_ctas,
                                      int staged_ctas, cudaStream_t stream) {
   CeStagePlan pl;
+  // chunks that the codec refuses (no multiple of 1024 values) are refused before a copy is planned for them
   if (!p.h2d || size_table == nullptr || p.chunk_bytes < kMinRowChunk || p.chunk_bytes % 2048 != 0 || layers_total != num_layers_ ||
       !plan(p, kMinRowBytes, kRowRampBytes, pl))
     return launch_kv_compress_bf16(p, size_table, layers_total, num_ctas, stream);

@@ -326,11 +326,15 @@ TransferGroup::Task TransferGroup::make_task(const int64_t* gpu_blocks, const in
 uint64_t TransferGroup::submit(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d,
                                int layer_start, int num_layers, int engine_override) {
   const Task t = make_task(gpu_blocks, cpu_blocks, n, h2d, layer_start, num_layers, engine_override);
+  enqueue(t);
+  return t.ticket;
+}
+
+void TransferGroup::enqueue(const Task& t) {
   for (auto& rk : ranks_) {
     { std::lock_guard<std::mutex> g(rk->mu); rk->q.push_back(t); }
     rk->cv.notify_one();
   }
-  return t.ticket;
 }
 
 OpResult TransferGroup::transfer(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d,
@@ -398,27 +402,9 @@ OpResult TransferGroup::wait(uint64_t ticket) {
 
 OpResult TransferGroup::transfer_refshape(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d,
                                           int num_ctas) {
-  if (n > opt_.max_blocks_per_op) throw std::invalid_argument("TransferGroup: op exceeds max_blocks_per_op");
-  Task t;
-  {
-    std::unique_lock<std::mutex> lk(mu_);
-    cv_.wait(lk, [&] { return !free_slots_.empty(); });
-    t.slot = free_slots_.back();
-    free_slots_.pop_back();
-    t.ticket = next_ticket_++;
-    t.rotate = op_counter_++;
-    Pending pd;
-    pd.remaining = (int)ranks_.size();
-    pd.slot = t.slot;
-    pending_[t.ticket] = pd;
-  }
-  std::memcpy(id_ring_ + ((size_t)t.slot * 2 + 0) * (size_t)opt_.max_blocks_per_op, gpu_blocks, (size_t)n * 8);
-  std::memcpy(id_ring_ + ((size_t)t.slot * 2 + 1) * (size_t)opt_.max_blocks_per_op, cpu_blocks, (size_t)n * 8);
-  t.n = n; t.h2d = h2d; t.layer_start = 0; t.num_layers = opt_.num_layers; t.engine = kEngineRefshape; t.refshape_ctas = num_ctas;
-  for (auto& rk : ranks_) {
-    { std::lock_guard<std::mutex> g(rk->mu); rk->q.push_back(t); }
-    rk->cv.notify_one();
-  }
+  Task t = make_task(gpu_blocks, cpu_blocks, n, h2d, 0, opt_.num_layers, kEngineRefshape);
+  t.refshape_ctas = num_ctas;
+  enqueue(t);
   return wait(t.ticket);
 }
 

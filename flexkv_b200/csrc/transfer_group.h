@@ -140,6 +140,7 @@ class TransferGroup {
   void rank_main(int r);
   Task make_task(const int64_t* gpu_blocks, const int64_t* cpu_blocks, int64_t n, bool h2d, int layer_start,
                  int num_layers, int engine_override);
+  void enqueue(const Task& t);
   Launched launch_task(int r, const Task& t, int slot);
   int retire_task(int r, const Launched& l, int slot, float& ms);
   void fill_params(int r, const Task& t, KvCopyParams& p, bool& skip) const;
