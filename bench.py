@@ -131,16 +131,20 @@ class ClockSampler:
 def kernel_desc(worker, env) -> dict:
     """Which kernel a worker launches and with what grid, for the bench line."""
     if hasattr(worker, "codec"):
-        pack = not worker.h2d
-        return {"kernel": f"kv_compress_kernel<{'pack' if pack else 'unpack'}> ({worker.codec})"
-                if worker.codec == "bf16_xp" else f"kv_quant_kernel<{'pack' if pack else 'unpack'}> ({worker.codec})",
-                "ctas": (int(worker.num_ctas) + 1) // 2 if worker.codec == "bf16_xp" else int(worker.num_ctas),
-                "threads": 256 if worker.codec == "bf16_xp" else 128,
-                "note": "two 128-thread tile pipelines per CTA" if worker.codec == "bf16_xp" else ""}
+        lossless, form = worker.codec == "bf16_xp", "unpack" if worker.h2d else "pack"
+        d = {"kernel": f"{'kv_compress_kernel' if lossless else 'kv_quant_fp8_kernel'}<{form}> ({worker.codec})",
+             "ctas": (int(worker.num_ctas) + 1) // 2 if lossless else int(worker.num_ctas), "threads": 256,
+             "note": "two 128-thread tile pipelines per CTA" if lossless else "one 256-thread tile pipeline per CTA"}
+        link = getattr(worker.strategy, "_link", None)
+        if link is not None:
+            # ops whose host blocks come in runs cross by copy engine, packed into or unpacked out of device staging
+            d["ops_through_copy_engines"] = int(link.staged_ops)
+            d["ctas_at_the_staging_buffer"] = (int(worker.staged_num_ctas) + 1) // 2 if lossless else d["ctas"]
+        return d
     ctas = env.transfer_num_cta_h2d if worker.h2d else env.transfer_num_cta_d2h
     eng = env.transfer_engine
     d = {"kernel": "kv_copy_bulk_kernel (cp.async.bulk ring)" if eng in ("tma", "auto", "") else f"engine={eng}",
-         "ctas": int(ctas), "threads": 64, "tile_bytes": int(env.transfer_tile_bytes), "engine": eng}
+         "ctas": int(ctas), "threads": 128 if int(env.transfer_tile_bytes) <= 16384 else 64, "tile_bytes": int(env.transfer_tile_bytes), "engine": eng}
     group = getattr(worker, "group", None)
     if eng in ("auto", "ce") and group is not None and hasattr(group, "ce_ops"):
         # the router sends an op to the copy engines when its host blocks form runs (gathered into device staging

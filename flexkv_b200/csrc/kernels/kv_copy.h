@@ -111,7 +111,7 @@ FKV_HD uint64_t kv_c_tensor(const KvCopyParams& p, int i) {
 }
 
 struct KvCopyLaunch {
-  int32_t num_ctas;     // persistent CTAs (each one bulk-copy pipeline)
+  int32_t num_ctas;     // persistent CTAs (four bulk-copy pipelines each, two with tiles above 16 KiB)
   int32_t tile_bytes;   // multiple of 16, <= 32 KiB
   int32_t engine;       // 0 = TMA bulk pipeline, 1 = SIMT vector ld/st
 };

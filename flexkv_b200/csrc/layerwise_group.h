@@ -51,7 +51,7 @@ struct LayerwiseOptions {
   uint32_t* size_table = nullptr;
   int size_table_layers = 0;
   int64_t size_table_rank_entries = 0;
-  int codec_pipelines = 64;   // 128-thread tile pipelines of the unpacking kernel (two per SM)
+  int codec_pipelines = 64;   // full-tile pipelines (128 threads) of the unpacking kernel, two to a CTA: half as many CTAs
 };
 
 struct LayerwiseResult {

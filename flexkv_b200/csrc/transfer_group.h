@@ -1,11 +1,13 @@
 // GPU<->host transfer executor for one tensor-parallel group.
 //
-// One persistent host thread, CUDA stream and mapped status word per GPU of
-// the group; an op (a list of gpu/cpu block-id pairs, a direction and a layer
-// range) is fanned out to every rank and joined. Block ids are written once
-// into a mapped pinned ring that all GPUs read directly, so an op costs one
-// kernel launch per GPU and no staging copies. Shared-KV (MLA) write modes
-// and the per-rank placement inside a host block follow the reference
+// One persistent host thread, CUDA stream and set of mapped status words per
+// GPU of the group; an op (a list of gpu/cpu block-id pairs, a direction and a
+// layer range) is fanned out to every rank and joined. A blocking op of a group
+// with one idle rank runs on the calling thread. Block ids are written once into
+// a mapped pinned ring that all GPUs read directly. An op is one kernel launch
+// per GPU, or, in a group of one GPU whose engine leaves the choice, driver
+// copies or the staged route of ce_copy.h. Shared-KV (MLA) write modes and the
+// per-rank placement inside a host block follow the reference
 // (csrc/tp_transfer_thread_group.cpp:199-381; flexkv/transfer/worker.py:1196-1204).
 #pragma once
 #include <atomic>

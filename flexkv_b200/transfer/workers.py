@@ -379,9 +379,10 @@ class QuantGpuHostWorker(TransferWorker):
         self.copy_engines = host_launch_cfg(GLOBAL_CONFIG_FROM_ENV, h2d, host)["engine"] >= _ENGINE_IDS["ce"]
         self.strategy = build_compressors(host, self.layers_total, self.regs[0].kv_dim, len(self.regs), self.shared)
         self.strategy.attach(self)
-        # Tile pipelines per launch (two share an SM in the lossless codec's kernel). Measured on B200 with
-        # Llama-3-8B blocks: 80 pipelines (40 SMs) put both directions on the link's plateau for SM-issued
-        # traffic; the fp8 kernel needs fewer (its CTAs are single pipelines)
+        # Width of a launch. Lossless: full-tile pipelines (128 threads), two to a CTA, so half as many CTAs; short tiles
+        # run four or eight to the same CTAs. Measured on B200 with Llama-3-8B blocks: 80 pipelines (40 SMs) put both
+        # directions on the link's plateau for SM-issued traffic. fp8: CTAs of 256 threads, one full tile or two or
+        # four short ones at a time.
         dflt = 80 if storage.host.quant == "bf16_xp" else (32 if h2d else 48)
         self.num_ctas = int(os.environ.get("FLEXKV_QUANT_NUM_CTA", dflt))
         # unpacking out of the staging buffer: twice the pipelines for a quarter of the time, so that the restore's
