@@ -28,13 +28,13 @@ def gpu_block_hashes(seqs: Sequence[torch.Tensor], tokens_per_block: int, namesp
         raise ValueError("gpu_block_hashes: every sequence must be a CUDA tensor on the device of the first")
     dev = seqs[0].device
     C = _native.C
-    s = stream if stream is not None else torch.cuda.current_stream(dev)
+    current = torch.cuda.current_stream(dev)
+    s = current if stream is None else stream
+    side = stream is not None and stream != current
     lens = [t.numel() for t in seqs]
     nblk = [n // tokens_per_block for n in lens]
     ns = namespace_prefix(namespace)
     out = torch.empty(sum(nblk), dtype=torch.int64, device=dev)
-    current = torch.cuda.current_stream(dev)
-    side = s != current
     if len(seqs) <= C.HASH_LIST_SEQS and (ns is None or ns.size <= C.HASH_LIST_NS) and max(lens) < 2**31:
         # addresses, lengths and prefix travel in the launch parameters; on the current stream the sequences are read
         # where they are

@@ -12,15 +12,16 @@ from __future__ import annotations
 from typing import Any, Dict
 
 from ... import _native
+from ...storage.storage_engine import host_register_chunk_bytes
 
 
-def codec_link(worker: Any, staging_bytes: int, min_op_bytes: int, min_chunk: int = 0):
+def codec_link(worker: Any, staging_bytes: int, min_op_bytes: int = 0, min_chunk: int = 0):
     """The native router of a worker's ops between kernel and copy engines, or None where every op belongs to the
-    kernel: an engine of the user's choice (FLEXKV_TRANSFER_ENGINE) or a host pool registered in parts
-    (``worker.copy_engines``), several ranks behind one op or one rank's slice of a wider block, which is not one span,
-    chunks below ``min_chunk`` bytes, or a pool that cannot hold an op of ``min_op_bytes``. The router takes twice
-    ``staging_bytes`` of GPU memory for its lifetime."""
-    if len(worker.regs) != 1 or not worker.copy_engines:
+    kernel: an engine of the user's choice (FLEXKV_TRANSFER_ENGINE), a host pool registered in parts, which a driver
+    copy must not straddle, several ranks behind one op (they read the same id arrays) or one rank's slice of a wider
+    block (which is not one span), chunks below ``min_chunk`` bytes, or a pool that cannot hold an op of
+    ``min_op_bytes``. The router takes twice ``staging_bytes`` of GPU memory for its lifetime."""
+    if len(worker.regs) != 1 or not worker.copy_engines or host_register_chunk_bytes():
         return None
     reg, host = worker.regs[0], worker.host
     if worker.kv_stride * reg.kv_dim * reg.num_layers != host.block_bytes or reg.chunk_bytes < min_chunk or \
