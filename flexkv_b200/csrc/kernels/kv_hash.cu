@@ -28,7 +28,7 @@ __device__ __forceinline__ uint64_t avalanche(uint64_t h) {
 // the accumulators of the previous one into digests. Segments are double-buffered, one barrier each.
 // Measured on B200 with the Python wrapper, before (four lanes did fetch, chain and digests in turn, inputs were
 // concatenated and three offset tables uploaded) -> now: 64 x 4096 tokens, 16 per block, GPU 351 -> 30 us, whole
-// call 343 -> 73 us; one 32K prompt 1764 -> 181 us; 64 x 4096 with one token per block 2710 -> 89 us; 8192 x 1024
+// call 343 -> 63 us; one 32K prompt 1764 -> 181 us; 64 x 4096 with one token per block 2710 -> 89 us; 8192 x 1024
 // tokens (flat form, eight sequences per CTA) 20.6 -> 14.6 ms, most of it concatenation.
 constexpr int kHashThreads = 128;
 constexpr int kHashHelpers = kHashThreads - 32;
